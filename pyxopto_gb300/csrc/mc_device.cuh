@@ -23,6 +23,7 @@
 #include <cfloat>
 #include "../../include/xopto_gb300.h"
 #include "portable_math.h"
+#include "exact_math.cuh"
 
 #ifndef MCGB_FAST_MATH
 #error "MCGB_FAST_MATH must be defined to 0 or 1"
@@ -40,15 +41,18 @@ MCGB_DEV float mc_div(float a, float b) { return __fdividef(a, b); }
 MCGB_DEV float mc_sqrt(float x) { return sqrtf(x); }
 MCGB_DEV float mc_rcp_length(float x2) { return rsqrtf(x2); }
 #else
-MCGB_DEV float mc_log(float x) { return pm_logf(x); }
-MCGB_DEV float mc_exp(float x) { return pm_expf(x); }
-MCGB_DEV float mc_pow(float x, float y) { return pm_powrf(x, y); }
+MCGB_DEV float mc_log(float x) { return em_log(x); }
+MCGB_DEV float mc_exp(float x) { return em_exp(x); }
+MCGB_DEV float mc_pow(float x, float y) { return em_powr(x, y); }
 MCGB_DEV float mc_cbrt(float x) { return pm_cbrtf(x); }
 MCGB_DEV void mc_sincos(float x, float *s, float *c) { pm_sincosf(x, s, c); }
-MCGB_DEV float mc_div(float a, float b) { return a / b; }
-MCGB_DEV float mc_sqrt(float x) { return sqrtf(x); }
+MCGB_DEV float mc_div(float a, float b) { return em_div(a, b); }
+MCGB_DEV float mc_sqrt(float x) { return em_sqrt(x); }
 /* mc_normalize_fpv3: k = 1/length (xopto/mcbase/kernel/mcbase.template.c:975-981) */
-MCGB_DEV float mc_rcp_length(float x2) { return 1.0f / sqrtf(x2); }
+MCGB_DEV float mc_rcp_length(float x2) {
+    if (x2 >= EM_LO && x2 <= EM_HI) return em_recip(em_sqrt_normal(x2));
+    return 1.0f / sqrtf(x2);
+}
 #endif
 
 struct f3 { float x, y, z; };
@@ -166,16 +170,47 @@ MCGB_DEV float step_factor(float inv_mut) { return -0.693147182f * inv_mut; }
 MCGB_DEV float sample_step(float u, float factor) { return __log2f(u) * factor; }
 #else
 MCGB_DEV float step_factor(float inv_mut) { return inv_mut; }
-MCGB_DEV float sample_step(float u, float factor) { return -mc_log(u) * factor; }
+MCGB_DEV float sample_step(float u, float factor) { return -em_log_uniform(u) * factor; }
 #endif
 
 /* scatter_direction + unconditional renormalisation,
-   xopto/mcbase/kernel/mcbase.template.c:1522-1555.  FAST mode divides by
-   sqrt(1 - uz^2) through one reciprocal square root. */
+   xopto/mcbase/kernel/mcbase.template.c:1522-1555, as one straight line: a
+   packet along z (the first scattering of a normally incident packet) takes
+   its direction by selects.  FAST mode divides by sqrt(1 - uz^2) through one
+   reciprocal square root; its multiply-adds are written out, so that the
+   bits do not depend on the code around the call.  EXACT mode tests the
+   operands of all its divisions and square roots at the end and repeats the
+   whole with IEEE operations when one is out of exact_math.cuh's range. */
+#if MCGB_FAST_MATH
 MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
     float sin_fi, cos_fi;
-    float sin_theta = mc_sqrt(1.0f - cos_theta * cos_theta);
+    float sin_theta = mc_sqrt(__fmaf_rn(-cos_theta, cos_theta, 1.0f));
     mc_sincos(fi, &sin_fi, &cos_fi);
+    float stcf = __fmul_rn(sin_theta, cos_fi);
+    float stsf = __fmul_rn(sin_theta, sin_fi);
+    float t = __fmaf_rn(-dir.z, dir.z, 1.0f);
+    float rk = rsqrtf(t);
+    float k = __fmul_rn(t, rk);
+    float nx = __fmaf_rn(__fmul_rn(stcf, dir.x), dir.z, -__fmul_rn(stsf, dir.y));
+    float ny = __fmaf_rn(stsf, dir.x, __fmul_rn(__fmul_rn(stcf, dir.y), dir.z));
+    float x = __fmaf_rn(dir.x, cos_theta, __fmul_rn(nx, rk));
+    float y = __fmaf_rn(dir.y, cos_theta, __fmul_rn(ny, rk));
+    float z = __fmaf_rn(dir.z, cos_theta, __fmul_rn(-stcf, k));
+    const bool along = fabsf(dir.z) >= 1.0f;
+    float zs = copysignf(cos_theta, dir.z * cos_theta);
+    x = along ? stcf : x;
+    y = along ? stsf : y;
+    z = along ? zs : z;
+    float r = rsqrtf(__fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x))));
+    dir.x = __fmul_rn(x, r);
+    dir.y = __fmul_rn(y, r);
+    dir.z = __fmul_rn(z, r);
+}
+#else
+static __device__ __noinline__ f3 scatter_direction_ieee(f3 dir, float cos_theta, float fi) {
+    float sin_fi, cos_fi;
+    float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
+    pm_sincosf(fi, &sin_fi, &cos_fi);
     float stcf = sin_theta * cos_fi;
     float stsf = sin_theta * sin_fi;
     float px = dir.x;
@@ -184,24 +219,44 @@ MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
         dir.y = stsf;
         dir.z = copysignf(cos_theta, dir.z * cos_theta);
     } else {
-#if MCGB_FAST_MATH
-        float t = 1.0f - dir.z * dir.z;
-        float rk = rsqrtf(t);
-        float k = t * rk;
-        dir.x = (stcf * px * dir.z - stsf * dir.y) * rk + px * cos_theta;
-        dir.y = (stcf * dir.y * dir.z + stsf * px) * rk + dir.y * cos_theta;
-#else
-        float k = mc_sqrt(1.0f - dir.z * dir.z);
-        dir.x = mc_div(stcf * px * dir.z - stsf * dir.y, k) + px * cos_theta;
-        dir.y = mc_div(stcf * dir.y * dir.z + stsf * px, k) + dir.y * cos_theta;
-#endif
+        float k = sqrtf(1.0f - dir.z * dir.z);
+        dir.x = (stcf * px * dir.z - stsf * dir.y) / k + px * cos_theta;
+        dir.y = (stcf * dir.y * dir.z + stsf * px) / k + dir.y * cos_theta;
         dir.z = (-stcf) * k + dir.z * cos_theta;
     }
-    float k = mc_rcp_length(dir.x * dir.x + dir.y * dir.y + dir.z * dir.z);
-    dir.x = dir.x * k;
-    dir.y = dir.y * k;
-    dir.z = dir.z * k;
+    float k = 1.0f / sqrtf(dir.x * dir.x + dir.y * dir.y + dir.z * dir.z);
+    return f3{dir.x * k, dir.y * k, dir.z * k};
 }
+
+MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
+    float sin_fi, cos_fi;
+    float st2 = 1.0f - cos_theta * cos_theta;
+    float sin_theta = em_sqrt_normal(st2);
+    em_sincos_azimuth(fi, &sin_fi, &cos_fi);   /* fi = 2 pi u */
+    float stcf = sin_theta * cos_fi;
+    float stsf = sin_theta * sin_fi;
+    /* |dir.z| < 1 unless along z: k lies in [2^-12, 1] */
+    float k = em_sqrt_normal(1.0f - dir.z * dir.z);
+    float yk = em_recip(k);
+    float nx = stcf * dir.x * dir.z - stsf * dir.y;
+    float ny = stcf * dir.y * dir.z + stsf * dir.x;
+    float x = em_quot(nx, k, yk) + dir.x * cos_theta;
+    float y = em_quot(ny, k, yk) + dir.y * cos_theta;
+    float z = (-stcf) * k + dir.z * cos_theta;
+    const bool along = fabsf(dir.z) >= 1.0f;
+    float zs = copysignf(cos_theta, dir.z * cos_theta);
+    x = along ? stcf : x;
+    y = along ? stsf : y;
+    z = along ? zs : z;
+    float r2 = x * x + y * y + z * z;
+    float r = em_recip(em_sqrt_normal(r2));
+    const float least = along ? 1.0f : fminf(fabsf(nx), fabsf(ny));
+    if (fminf(fminf(st2, least), r2) >= EM_LO && r2 <= EM_HI)
+        dir = f3{x * r, y * r, z * r};
+    else
+        dir = scatter_direction_ieee(dir, cos_theta, fi);
+}
+#endif
 
 /* Phase-function constants of one layer/material, precomputed once per
    kernel with the same float operations the per-step formulas use, so the
@@ -210,7 +265,9 @@ MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
      Hg:  pf0 = (g, 1 - g*g, 1 + g*g, 2*g)
      Gk:  pf0 = (g, a, -inv_a, a1), pf1 = (a2, 1 + g*g, 2*g, (1 - g)/(1 + g))
      Lut: pf0 = (a, b, c, (float)(N - 1)), pf1 = (offset, N - 1) as int bits
-   FAST math stores 1/(2g) in place of 2g and multiplies (pf_div2g). */
+   FAST math stores 1/(2g) in place of 2g and multiplies (pf_div2g).  EXACT
+   math adds pf1 = (RN(1/(2g)), 1 where exact_math.cuh covers every division
+   by 1 + g (2u - 1) and 2g, else 0) to Hg. */
 #if MCGB_FAST_MATH
 MCGB_DEV float pf_2g(float g) { return 1.0f / (2.0f * g); }
 MCGB_DEV float pf_div2g(float x, float c) { return x * c; }
@@ -222,7 +279,12 @@ MCGB_DEV void pf_prepare(int kind, const McgbPf &pf, float4 &pf0, float4 &pf1) {
     if (kind == MCGB_PF_HG) {
         float g = pf.p[0];
         pf0 = make_float4(g, 1.0f - g * g, 1.0f + g * g, pf_2g(g));
+#if MCGB_FAST_MATH
         pf1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#else
+        const bool plain = fabsf(g) >= 9.3132257461547852e-10f && fabsf(g) <= 0.9999990463256836f;
+        pf1 = make_float4(plain ? em_recip(2.0f * g) : 0.0f, plain ? 1.0f : 0.0f, 0.0f, 0.0f);
+#endif
     } else if (kind == MCGB_PF_GK) {
         float g = pf.p[0];
         pf0 = make_float4(g, pf.p[1], -pf.p[2], pf.p[3]);
@@ -266,6 +328,32 @@ MCGB_DEV float pf_sample(const float4 &pf0, const float4 &pf1, const float *lut,
         return cos_theta;
     }
     *azimuth = 6.28318548f * rng.next();
+#if !MCGB_FAST_MATH
+    /* Hg and Gk as a straight line; the reference's expressions below serve
+       the parameters and operands that exact_math.cuh does not cover. */
+    if (PF == MCGB_PF_HG) {
+        Rng next = rng;
+        float den = 1.0f + pf0.x * (2.0f * next.next() - 1.0f);
+        float k = em_quot(pf0.y, den, em_recip(den));
+        float cos_theta = em_quot(pf0.z - k * k, pf0.w, pf1.x);
+        if (pf1.y != 0.0f) {
+            rng = next;
+            return fmaxf(fminf(cos_theta, 1.0f), -1.0f);
+        }
+    } else if (PF == MCGB_PF_GK) {
+        Rng next = rng;
+        float base = pf0.w * next.next() + pf1.x;
+        float e = pf0.z * em_log_normal(base);
+        float tmp = pf1.y - em_exp_mid(e);
+        float cos_theta = em_quot(tmp, pf1.z, em_recip(pf1.z));
+        /* tmp is 0 or at least 2^-24 of its larger term, below 2^117 */
+        if (__float_as_uint(base) - 0x00800000u < 0x7f000000u && fabsf(e) <= 40.0f && pf0.y != 0.0f &&
+            fabsf(pf1.z) >= EM_LO) {
+            rng = next;
+            return fminf(fmaxf(cos_theta, -1.0f), 1.0f);
+        }
+    }
+#endif
     if (PF == MCGB_PF_HG) {
         float g = pf0.x;
         float k = mc_div(pf0.y, 1.0f + g * (2.0f * rng.next() - 1.0f));
@@ -591,9 +679,10 @@ struct FluenceCache {
         sum = 0;
     }
     /* Branch-free: the reduction of the previous voxel's sum is predicated
-       on a change of voxel, so lanes of a warp do not diverge around it. */
-    __device__ __forceinline__ void add(uint32_t i, uint32_t w) {
-        const bool miss = i != index;
+       on a change of voxel, and a deposit outside the grid (in = false)
+       leaves the cache as it is, so lanes of a warp do not diverge. */
+    __device__ __forceinline__ void add(bool in, uint32_t i, uint32_t w) {
+        const bool miss = in && i != index;
         const int fire = (miss && sum != 0ull) ? 1 : 0;
         unsigned long long *addr = (unsigned long long *)(base + index);
         asm volatile(
@@ -603,7 +692,7 @@ struct FluenceCache {
             "l"((unsigned long long)sum), "r"(fire)
             : "memory");
         index = miss ? i : index;
-        sum = (miss ? 0ull : sum) + w;
+        sum = (miss ? 0ull : sum) + (in ? w : 0u);
     }
 };
 
@@ -633,12 +722,11 @@ MCGB_DEV void fluence_deposit(const McgbFluence &fl, const f3 &pos, float weight
     uint32_t jx = (uint32_t)__float2int_rd(ix);
     uint32_t jy = (uint32_t)__float2int_rd(iy);
     uint32_t jz = (uint32_t)__float2int_rd(iz);
-    if (jx < fl.shape[0] && jy < fl.shape[1] && jz < fl.shape[2]) {
-        uint32_t index = (jz * fl.shape[1] + jy) * fl.shape[0] + jx;
-        if (RATE && fl.kind == MCGB_FLUENCE_RATE) weight *= (mua != 0.0f) ? mc_div(1.0f, mua) : 0.0f;
-        uint32_t w = (uint32_t)(weight * (float)fl.k + 0.5f);
-        cache.add(index, w);
-    }
+    const bool in = jx < fl.shape[0] && jy < fl.shape[1] && jz < fl.shape[2];
+    uint32_t index = (jz * fl.shape[1] + jy) * fl.shape[0] + jx;
+    if (RATE && fl.kind == MCGB_FLUENCE_RATE) weight *= (mua != 0.0f) ? mc_div(1.0f, mua) : 0.0f;
+    uint32_t w = (uint32_t)(weight * (float)fl.k + 0.5f);
+    cache.add(in, index, w);
 }
 
 /* Event bits, xopto/mcbase/kernel/mcbase.template.h:640-660 */
