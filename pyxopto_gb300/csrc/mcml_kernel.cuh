@@ -24,6 +24,7 @@
 #pragma once
 #include "mc_device.cuh"
 #include "batch_rng.h"
+#include "work_share.cuh"
 
 namespace MCGB_NS {
 
@@ -481,7 +482,7 @@ static __device__ __forceinline__ MlCtx mcml_ctx(const McgbMcmlConfig &c, const 
     return x;
 }
 
-template <bool SIMPLE>
+template <bool SIMPLE, bool XTRA>
 static __device__ __forceinline__ void mcml_begin(const McgbMcmlConfig &c, const McgbBuffers &b,
                                                   const MlCtx &x, MlPacket &s, Rng &rng, uint64_t p) {
     s.p = p;
@@ -490,13 +491,14 @@ static __device__ __forceinline__ void mcml_begin(const McgbMcmlConfig &c, const
     s.steps = 0;
     s.events = MCGB_EV_LAUNCH;
     mcml_launch<SIMPLE>(c, x.L, x.lut, rng, s.pos, s.dir, s.w, s.layer, b.accumulator);
-    if (x.use_trace && (c.trace.flags & MCGB_TRACE_START))
+    if (XTRA && x.use_trace && (c.trace.flags & MCGB_TRACE_START))
         trace_event(c.trace, s.p, s.trace_count, s.events, s.pos, s.dir, s.w, s.opl, b.float_buffer);
 }
 
+template <bool XTRA>
 static __device__ __forceinline__ void mcml_end(const McgbMcmlConfig &c, const McgbBuffers &b,
                                                 const MlCtx &x, const MlPacket &s) {
-    if (x.use_trace) b.int_buffer[c.trace.count_offset + s.p] = (int32_t)s.trace_count;
+    if (XTRA && x.use_trace) b.int_buffer[c.trace.count_offset + s.p] = (int32_t)s.trace_count;
 }
 
 /* The end of a step: rmax (mcml.template.c:759-763), the trace event and the
@@ -751,18 +753,18 @@ mcml_transport_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffer
     uint64_t steps = 0, packets = 0;
     uint32_t iter = 0, status = 0;
     MlPacket s;
-    mcml_begin<false>(c, b, x, s, rng, t);
+    mcml_begin<false, true>(c, b, x, s, rng, t);
     for (;;) {
         if (mcml_step<PF, METHOD, FLU, true>(c, b, x, s, rng, fcache, status)) {
             ++packets;
             steps += s.steps;
-            mcml_end(c, b, x, s);
+            mcml_end<true>(c, b, x, s);
             uint64_t p = s.p + T;
             if (p >= c.num_packets) {
                 s.steps = 0;
                 break;
             }
-            mcml_begin<false>(c, b, x, s, rng, p);
+            mcml_begin<false, true>(c, b, x, s, rng, p);
         }
         if (((++iter) & 1023u) == 0) {
             if (globaltimer_ns() > t_deadline) { status |= MCGB_STATUS_TIMEOUT; break; }
@@ -777,21 +779,43 @@ mcml_transport_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffer
 
 #define MCGB_FULL_MASK 0xffffffffu
 
+/* Threads per block of the dynamic kernel: the warps that merge their last
+   packets, half of the SM's 32 resident warps at 64 registers.  Against
+   blocks of 128 and 256 threads: 1e6 packets of the 10 mm slab 1.41 ms
+   (1.56, 1.46), 1e7 of the skin stack 45.9 ms (46.9, 46.2), 1e6 7.5 ms
+   (8.4, 7.7). */
+#define ML_BLOCK 512
+
+/* Everything of a packet that moves between warps (work_share.cuh). */
+template <bool XTRA, class IO>
+static __device__ __forceinline__ void mcml_state(IO &io, MlPacket &s, Rng &rng) {
+    io(s.pos.x); io(s.pos.y); io(s.pos.z);
+    io(s.dir.x); io(s.dir.y); io(s.dir.z);
+    io(s.w); io(s.layer); io(s.steps);
+    io(rng.x); io(rng.a);
+    if (XTRA) {
+        io(s.opl); io(s.trace_count); io(s.events); io(s.p);
+    }
+}
+typedef WsExchange<17, ML_BLOCK / 32> MlExchange;
+
 /* DYNAMIC scheduling: persistent warps refill idle lanes packet by packet
    from the queue counters[MCGB_CNT_QUEUE]; packet p runs on the stream of
    (seed, packet_offset + p). */
 template <int PF, int METHOD, bool FLU, bool XTRA, bool SIMPLE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(ML_BLOCK, 2)
 mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers b,
                     uint64_t deadline_ns, int lut_in_smem, uint32_t packets_per_item) {
     __shared__ MlSmem sm;
+    __shared__ MlExchange share;
     extern __shared__ float s_lut[];
+    ws_init(share);
     const float *lut = mcml_stage<PF>(c, b, sm, s_lut, lut_in_smem);
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t t_deadline = globaltimer_ns() + deadline_ns;
     const MlCtx x = mcml_ctx(c, sm.layers, lut);
     const uint64_t N = c.num_packets;
-    const uint64_t B = packets_per_item;
+    const uint32_t warps = gridDim.x * (ML_BLOCK / 32);
     unsigned long long *queue = (unsigned long long *)(b.counters + MCGB_CNT_QUEUE);
     uint64_t item_next = 0, item_end = 0;   /* warp-uniform */
     bool more = true, active = false;
@@ -800,20 +824,15 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
     uint64_t steps = 0, packets = 0;
     uint32_t iter = 0, status = 0;
     MlPacket s;
-    s.steps = 0;
     for (;;) {
         uint32_t need = __ballot_sync(MCGB_FULL_MASK, !active);
         while (need && more) {
             if (item_next >= item_end) {
-                unsigned long long item = 0;
-                if (lane == 0) item = atomicAdd(queue, 1ull);
-                item = __shfl_sync(MCGB_FULL_MASK, item, 0);
-                item_next = (uint64_t)item * B;
+                ws_fetch(queue, N, packets_per_item, warps, __popc(need), item_next, item_end);
                 if (item_next >= N) {
                     more = false;
                     break;
                 }
-                item_end = min(item_next + B, N);
             }
             uint32_t avail = (uint32_t)min(item_end - item_next, (uint64_t)32);
             uint32_t rank = __popc(need & ((1u << lane) - 1u));
@@ -824,14 +843,14 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
                 uint32_t as;
                 br_packet_stream(c.opt.seed, 0u, c.opt.packet_offset + p, b.rng_a, c.num_streams, &xs, &as);
                 rng = Rng{xs, as};
-                mcml_begin<SIMPLE>(c, b, x, s, rng, p);
+                mcml_begin<SIMPLE, XTRA>(c, b, x, s, rng, p);
                 active = true;
             }
             uint32_t taken = __ballot_sync(MCGB_FULL_MASK, mine);
             item_next += __popc(taken);
             need &= ~taken;
         }
-        if (!__any_sync(MCGB_FULL_MASK, active)) break;
+        if (!more && !ws_share(share, active, [&](auto &io) { mcml_state<XTRA>(io, s, rng); })) break;
         /* sixteen steps between refills; two steps per loop iteration give
            the scheduler both bodies (+0.9 % on the layered stack) */
 #pragma unroll 2
@@ -839,8 +858,7 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
             if (active && mcml_step<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status)) {
                 ++packets;
                 steps += s.steps;
-                s.steps = 0;
-                mcml_end(c, b, x, s);
+                mcml_end<XTRA>(c, b, x, s);
                 active = false;
             }
         }
@@ -854,13 +872,14 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
             stop = __shfl_sync(MCGB_FULL_MASK, stop, 0);
             if (stop) {
                 status |= stop;
+                ws_leave(share);
                 break;
             }
         }
     }
-    steps += s.steps;
+    if (active) steps += s.steps;
     if (FLU) fcache.flush();
-    mc_finish(b, steps, packets, status, packets > 0);
+    warp_finish(b, steps, packets, status);
 }
 
 }  // namespace MCGB_NS

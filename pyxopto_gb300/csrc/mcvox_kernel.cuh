@@ -11,6 +11,7 @@
 #pragma once
 #include "mc_device.cuh"
 #include "batch_rng.h"
+#include "work_share.cuh"
 
 namespace MCGB_NS {
 
@@ -430,7 +431,7 @@ static __device__ __forceinline__ MvCtx mcvox_ctx(const McgbMcvoxConfig &c, cons
     return x;
 }
 
-template <bool SIMPLE>
+template <bool SIMPLE, bool XTRA>
 static __device__ __forceinline__ void mcvox_begin(const McgbMcvoxConfig &c, const McgbBuffers &b,
                                                    const MvCtx &x, MvPacket &s, Rng &rng, uint64_t p,
                                                    f3 prev_pos) {
@@ -444,13 +445,14 @@ static __device__ __forceinline__ void mcvox_begin(const McgbMcvoxConfig &c, con
     s.k = MCGB_FAST_MATH ? mv_cube_k(x, s.vi) : 0;
     s.free = MCGB_FAST_MATH ? mv_ball(x, s.k) : 0.0f;
     s.pend = -1.0f;
-    if (x.use_trace && (c.trace.flags & MCGB_TRACE_START))
+    if (XTRA && x.use_trace && (c.trace.flags & MCGB_TRACE_START))
         trace_event(c.trace, s.p, s.trace_count, s.events, s.pos, s.dir, s.w, s.opl, b.float_buffer);
 }
 
+template <bool XTRA>
 static __device__ __forceinline__ void mcvox_end(const McgbMcvoxConfig &c, const McgbBuffers &b,
                                                  const MvCtx &x, const MvPacket &s) {
-    if (x.use_trace) b.int_buffer[c.trace.count_offset + s.p] = (int32_t)s.trace_count;
+    if (XTRA && x.use_trace) b.int_buffer[c.trace.count_offset + s.p] = (int32_t)s.trace_count;
 }
 
 /* One step of McKernel (mcvox), xopto/mcvox/kernel/mcvox.template.c:760-1038.
@@ -708,18 +710,18 @@ mcvox_transport_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuff
     uint32_t iter = 0, status = 0;
     MvPacket s;
     s.pos = f3{0.0f, 0.0f, 0.0f};
-    mcvox_begin<false>(c, b, x, s, rng, t, s.pos);
+    mcvox_begin<false, true>(c, b, x, s, rng, t, s.pos);
     for (;;) {
         if (mcvox_step<PF, METHOD, FLU, true>(c, b, x, s, rng, fcache, status)) {
             ++packets;
             steps += s.steps;
-            mcvox_end(c, b, x, s);
+            mcvox_end<true>(c, b, x, s);
             uint64_t p = s.p + T;
             if (p >= c.num_packets) {
                 s.steps = 0;
                 break;
             }
-            mcvox_begin<false>(c, b, x, s, rng, p, s.pos);
+            mcvox_begin<false, true>(c, b, x, s, rng, p, s.pos);
         }
         if (((++iter) & 1023u) == 0) {
             if (globaltimer_ns() > t_deadline) { status |= MCGB_STATUS_TIMEOUT; break; }
@@ -732,13 +734,36 @@ mcvox_transport_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuff
     mv_finish(b, steps, packets, status, true);
 }
 
+/* Threads per block of the dynamic kernel: the warps that merge their last
+   packets.  The plain Line and GaussianBeam kernels take 64 registers by
+   themselves; asking for them (four blocks) cost 4 % on the skin and vessel
+   grid.  The others are held to 80 (24 warps). */
+#define MV_BLOCK 256
+
+/* Everything of a packet that moves between warps (work_share.cuh). */
+template <bool XTRA, class IO>
+static __device__ __forceinline__ void mcvox_state(IO &io, MvPacket &s, Rng &rng) {
+    io(s.pos.x); io(s.pos.y); io(s.pos.z);
+    io(s.dir.x); io(s.dir.y); io(s.dir.z);
+    io(s.vi.x); io(s.vi.y); io(s.vi.z);
+    io(s.mat); io(s.w); io(s.steps);
+    io(s.free); io(s.k); io(s.pend);   /* constants without free flight */
+    io(rng.x); io(rng.a);
+    if (XTRA) {
+        io(s.opl); io(s.trace_count); io(s.events); io(s.p);
+    }
+}
+typedef WsExchange<23, MV_BLOCK / 32> MvExchange;
+
 /* DYNAMIC scheduling (per-packet streams, warp refill). */
 template <int PF, int METHOD, bool FLU, bool XTRA, bool SIMPLE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(MV_BLOCK, SIMPLE && !XTRA ? 1 : 3)
 mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffers b,
                      uint64_t deadline_ns, int lut_in_smem, uint32_t packets_per_item) {
     __shared__ MvSmem sm;
+    __shared__ MvExchange share;
     extern __shared__ float s_lut[];
+    ws_init(share);
     const float *lut = mcvox_stage<PF>(c, b, sm, s_lut, lut_in_smem);
     /* the phased loop: FAST free flight in the plain kernels */
     constexpr bool PHASED = MCGB_FAST_MATH && METHOD != MCGB_METHOD_MICROSCOPIC_BEER_LAMBERT && !XTRA;
@@ -746,7 +771,7 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
     const uint64_t t_deadline = globaltimer_ns() + deadline_ns;
     const MvCtx x = mcvox_ctx(c, b, sm.materials, lut);
     const uint64_t N = c.num_packets;
-    const uint64_t B = packets_per_item;
+    const uint32_t warps = gridDim.x * (MV_BLOCK / 32);
     unsigned long long *queue = (unsigned long long *)(b.counters + MCGB_CNT_QUEUE);
     uint64_t item_next = 0, item_end = 0;
     bool more = true, active = false;
@@ -755,20 +780,15 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
     uint64_t steps = 0, packets = 0;
     uint32_t iter = 0, status = 0;
     MvPacket s;
-    s.steps = 0;
     for (;;) {
         uint32_t need = __ballot_sync(0xffffffffu, !active);
         while (need && more) {
             if (item_next >= item_end) {
-                unsigned long long item = 0;
-                if (lane == 0) item = atomicAdd(queue, 1ull);
-                item = __shfl_sync(0xffffffffu, item, 0);
-                item_next = (uint64_t)item * B;
+                ws_fetch(queue, N, packets_per_item, warps, __popc(need), item_next, item_end);
                 if (item_next >= N) {
                     more = false;
                     break;
                 }
-                item_end = min(item_next + B, N);
             }
             uint32_t avail = (uint32_t)min(item_end - item_next, (uint64_t)32);
             uint32_t rank = __popc(need & ((1u << lane) - 1u));
@@ -779,14 +799,14 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
                 uint32_t as;
                 br_packet_stream(c.opt.seed, 0u, c.opt.packet_offset + p, b.rng_a, c.num_streams, &xs, &as);
                 rng = Rng{xs, as};
-                mcvox_begin<SIMPLE>(c, b, x, s, rng, p, f3{0.0f, 0.0f, 0.0f});
+                mcvox_begin<SIMPLE, XTRA>(c, b, x, s, rng, p, f3{0.0f, 0.0f, 0.0f});
                 active = true;
             }
             uint32_t taken = __ballot_sync(0xffffffffu, mine);
             item_next += __popc(taken);
             need &= ~taken;
         }
-        if (!__any_sync(0xffffffffu, active)) break;
+        if (!more && !ws_share(share, active, [&](auto &io) { mcvox_state<XTRA>(io, s, rng); })) break;
         /* 32 steps between refills (+0.6 % against 16 on the skin and
            vessel grid); the step body is not unrolled (two bodies per
            iteration cost 10 % here) */
@@ -809,16 +829,14 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
                     if (mcvox_move<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status, step)) {
                         ++packets;
                         steps += s.steps;
-                        s.steps = 0;
-                        mcvox_end(c, b, x, s);
+                        mcvox_end<XTRA>(c, b, x, s);
                         active = false;
                     }
                 }
             } else if (active && mcvox_step<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status)) {
                 ++packets;
                 steps += s.steps;
-                s.steps = 0;
-                mcvox_end(c, b, x, s);
+                mcvox_end<XTRA>(c, b, x, s);
                 active = false;
             }
         }
@@ -832,13 +850,14 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
             stop = __shfl_sync(0xffffffffu, stop, 0);
             if (stop) {
                 status |= stop;
+                ws_leave(share);
                 break;
             }
         }
     }
-    steps += s.steps;
+    if (active) steps += s.steps;
     if (FLU) fcache.flush();
-    mv_finish(b, steps, packets, status, packets > 0);
+    warp_finish(b, steps, packets, status);
 }
 
 }  // namespace MCGB_NS

@@ -17,6 +17,7 @@
 #define MCGB_DYNAMIC_KERNEL mcml_dynamic_kernel
 #define MCGB_CFG McgbMcmlConfig
 #define MCGB_LAUNCH launch_mcml
+#define MCGB_BLOCK ML_BLOCK
 #define MCGB_OCCUPANCY occupancy_mcml
 #define MCGB_SELECT_STATIC select_static_mcml
 #else
@@ -25,6 +26,7 @@
 #define MCGB_DYNAMIC_KERNEL mcvox_dynamic_kernel
 #define MCGB_CFG McgbMcvoxConfig
 #define MCGB_LAUNCH launch_mcvox
+#define MCGB_BLOCK MV_BLOCK
 #define MCGB_OCCUPANCY occupancy_mcvox
 #define MCGB_SELECT_STATIC select_static_mcvox
 #endif
@@ -125,9 +127,8 @@ cudaError_t MCGB_LAUNCH(const MCGB_CFG &cfg, const McgbBuffers &buf, cudaStream_
     }
     unsigned grid = shape.grid, block = shape.block;
     if (sched == MCGB_SCHED_DYNAMIC) {
-        /* persistent: as many 128-thread blocks as stay resident (the
-           dynamic kernels are compiled for 128-thread blocks) */
-        block = 128;
+        /* persistent: as many blocks as stay resident */
+        block = MCGB_BLOCK;
         int dev = 0, sms = 0, bps = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -136,15 +137,8 @@ cudaError_t MCGB_LAUNCH(const MCGB_CFG &cfg, const McgbBuffers &buf, cudaStream_
         if (bps < 1) return cudaErrorInvalidConfiguration;
         grid = (unsigned)(sms * bps);
     }
-    /* dynamic scheduling: packets per queue item; by default at least 4
-       items per warp of the grid (so that short runs still spread over every
-       warp), at most 128 (one queue access per 128 packets in long runs) */
+    /* dynamic scheduling: packets per queue visit, 0 = by what is left (ws_fetch) */
     uint32_t items = cfg.opt.packets_per_item;
-    if (items == 0) {
-        uint64_t warps = (uint64_t)grid * (block / 32u);
-        uint64_t b = cfg.num_packets / (warps * 4u);
-        items = (uint32_t)(b < 1 ? 1 : (b > 128 ? 128 : b));
-    }
     McgbBuffers b = buf;
     uint64_t deadline = shape.deadline_ns;
     int lut = shape.lut_in_smem;
