@@ -178,10 +178,12 @@ MCGB_DEV float sample_step(float u, float factor) { return -em_log_uniform(u) * 
    packet along z (the first scattering of a normally incident packet) takes
    its direction by selects.  FAST mode divides by sqrt(1 - uz^2) through one
    reciprocal square root; its multiply-adds are written out, so that the
-   bits do not depend on the code around the call.  EXACT mode tests the
-   operands of all its divisions and square roots at the end and repeats the
-   whole with IEEE operations when one is out of exact_math.cuh's range. */
+   bits do not depend on the code around the call (YX: the squared length
+   begins with y, as in the batched engine, instead of x).  EXACT mode tests
+   the operands of all its divisions and square roots at the end and repeats
+   the whole with IEEE operations when one is out of exact_math.cuh's range. */
 #if MCGB_FAST_MATH
+template <bool YX = false>
 MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
     float sin_fi, cos_fi;
     float sin_theta = mc_sqrt(__fmaf_rn(-cos_theta, cos_theta, 1.0f));
@@ -201,7 +203,7 @@ MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
     x = along ? stcf : x;
     y = along ? stsf : y;
     z = along ? zs : z;
-    float r = rsqrtf(__fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x))));
+    float r = rsqrtf(__fmaf_rn(z, z, YX ? __fmaf_rn(x, x, __fmul_rn(y, y)) : __fmaf_rn(y, y, __fmul_rn(x, x))));
     dir.x = __fmul_rn(x, r);
     dir.y = __fmul_rn(y, r);
     dir.z = __fmul_rn(z, r);
@@ -228,6 +230,7 @@ static __device__ __noinline__ f3 scatter_direction_ieee(f3 dir, float cos_theta
     return f3{dir.x * k, dir.y * k, dir.z * k};
 }
 
+template <bool YX = false>
 MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
     float sin_fi, cos_fi;
     float st2 = 1.0f - cos_theta * cos_theta;
@@ -770,7 +773,7 @@ MCGB_DEV uint64_t globaltimer_ns() {
 /* Run totals of one warp: the lanes' counts are added in the warp and lane 0
    sends one reduction per counter.  One reduction per thread and counter
    queued 389,120 reductions on two addresses, about 0.15 ms of every run. */
-MCGB_DEV void warp_finish(const McgbBuffers &b, uint64_t steps, uint64_t packets, uint32_t status) {
+MCGB_DEV void warp_finish(uint64_t *counters, uint64_t steps, uint64_t packets, uint32_t status) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t threads = __popc(__ballot_sync(0xffffffffu, packets > 0));
 #pragma unroll
@@ -780,10 +783,10 @@ MCGB_DEV void warp_finish(const McgbBuffers &b, uint64_t steps, uint64_t packets
     }
     status = __reduce_or_sync(0xffffffffu, status);
     if (lane != 0) return;
-    if (steps) atomicAdd((unsigned long long *)(b.counters + MCGB_CNT_STEPS), (unsigned long long)steps);
+    if (steps) atomicAdd((unsigned long long *)(counters + MCGB_CNT_STEPS), (unsigned long long)steps);
     if (threads) {
-        atomicAdd((unsigned long long *)(b.counters + MCGB_CNT_PACKETS), (unsigned long long)packets);
-        atomicAdd((unsigned long long *)(b.counters + MCGB_CNT_THREADS), (unsigned long long)threads);
+        atomicAdd((unsigned long long *)(counters + MCGB_CNT_PACKETS), (unsigned long long)packets);
+        atomicAdd((unsigned long long *)(counters + MCGB_CNT_THREADS), (unsigned long long)threads);
     }
-    if (status) atomicOr((unsigned long long *)(b.counters + MCGB_CNT_STATUS), (unsigned long long)status);
+    if (status) atomicOr((unsigned long long *)(counters + MCGB_CNT_STATUS), (unsigned long long)status);
 }

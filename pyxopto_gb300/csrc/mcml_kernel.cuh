@@ -797,7 +797,7 @@ static __device__ __forceinline__ void mcml_state(IO &io, MlPacket &s, Rng &rng)
         io(s.opl); io(s.trace_count); io(s.events); io(s.p);
     }
 }
-typedef WsExchange<17, ML_BLOCK / 32> MlExchange;
+typedef WsExchange<17, ML_BLOCK / 32, 1, 8> MlExchange;
 
 /* DYNAMIC scheduling: persistent warps refill idle lanes packet by packet
    from the queue counters[MCGB_CNT_QUEUE]; packet p runs on the stream of
@@ -816,6 +816,7 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
     const MlCtx x = mcml_ctx(c, sm.layers, lut);
     const uint64_t N = c.num_packets;
     const uint32_t warps = gridDim.x * (ML_BLOCK / 32);
+    const bool takes = ws_takes(share, N, packets_per_item, warps);
     unsigned long long *queue = (unsigned long long *)(b.counters + MCGB_CNT_QUEUE);
     uint64_t item_next = 0, item_end = 0;   /* warp-uniform */
     bool more = true, active = false;
@@ -825,10 +826,10 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
     uint32_t iter = 0, status = 0;
     MlPacket s;
     for (;;) {
-        uint32_t need = __ballot_sync(MCGB_FULL_MASK, !active);
+        uint32_t need = __ballot_sync(MCGB_FULL_MASK, takes && !active);
         while (need && more) {
             if (item_next >= item_end) {
-                ws_fetch(queue, N, packets_per_item, warps, __popc(need), item_next, item_end);
+                ws_fetch(queue, N, packets_per_item, 128, warps, __popc(need), item_next, item_end);
                 if (item_next >= N) {
                     more = false;
                     break;
@@ -879,7 +880,7 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
     }
     if (active) steps += s.steps;
     if (FLU) fcache.flush();
-    warp_finish(b, steps, packets, status);
+    warp_finish(b.counters, steps, packets, status);
 }
 
 }  // namespace MCGB_NS

@@ -736,8 +736,8 @@ mcvox_transport_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuff
 
 /* Threads per block of the dynamic kernel: the warps that merge their last
    packets.  The plain Line and GaussianBeam kernels take 64 registers by
-   themselves; asking for them (four blocks) cost 4 % on the skin and vessel
-   grid.  The others are held to 80 (24 warps). */
+   themselves; with a minimum of four blocks they lost 4 % on the skin and
+   vessel grid, with a minimum of one (76 registers) 30 %. */
 #define MV_BLOCK 256
 
 /* Everything of a packet that moves between warps (work_share.cuh). */
@@ -753,11 +753,11 @@ static __device__ __forceinline__ void mcvox_state(IO &io, MvPacket &s, Rng &rng
         io(s.opl); io(s.trace_count); io(s.events); io(s.p);
     }
 }
-typedef WsExchange<23, MV_BLOCK / 32> MvExchange;
+typedef WsExchange<23, MV_BLOCK / 32, 2, 2> MvExchange;
 
 /* DYNAMIC scheduling (per-packet streams, warp refill). */
 template <int PF, int METHOD, bool FLU, bool XTRA, bool SIMPLE>
-__global__ void __launch_bounds__(MV_BLOCK, SIMPLE && !XTRA ? 1 : 3)
+__global__ void __launch_bounds__(MV_BLOCK)
 mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffers b,
                      uint64_t deadline_ns, int lut_in_smem, uint32_t packets_per_item) {
     __shared__ MvSmem sm;
@@ -772,6 +772,7 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
     const MvCtx x = mcvox_ctx(c, b, sm.materials, lut);
     const uint64_t N = c.num_packets;
     const uint32_t warps = gridDim.x * (MV_BLOCK / 32);
+    const bool takes = ws_takes(share, N, packets_per_item, warps);
     unsigned long long *queue = (unsigned long long *)(b.counters + MCGB_CNT_QUEUE);
     uint64_t item_next = 0, item_end = 0;
     bool more = true, active = false;
@@ -781,10 +782,10 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
     uint32_t iter = 0, status = 0;
     MvPacket s;
     for (;;) {
-        uint32_t need = __ballot_sync(0xffffffffu, !active);
+        uint32_t need = __ballot_sync(0xffffffffu, takes && !active);
         while (need && more) {
             if (item_next >= item_end) {
-                ws_fetch(queue, N, packets_per_item, warps, __popc(need), item_next, item_end);
+                ws_fetch(queue, N, packets_per_item, 128, warps, __popc(need), item_next, item_end);
                 if (item_next >= N) {
                     more = false;
                     break;
@@ -857,7 +858,7 @@ mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffer
     }
     if (active) steps += s.steps;
     if (FLU) fcache.flush();
-    warp_finish(b, steps, packets, status);
+    warp_finish(b.counters, steps, packets, status);
 }
 
 }  // namespace MCGB_NS

@@ -45,27 +45,35 @@ struct WsLoad {
     }
 };
 
-template <int WORDS, int WARPS>
+/* KEEP and SHARE by how much the kernel's steps diverge.  Layered: 1 and 8
+   (four warps of an SM in the shortest runs); voxelized, where the lanes
+   split between flights and walls: 2 and 2 (16 warps).  5e3 packets of the
+   voxel grid with 1 and 1000 (all lanes of a warp) 2.1 ms, with 2 and 2 1.25
+   ms (1.23 before warps merged); 3e3 of the slab with 1000 0.33, with 8 0.30
+   ms (0.55 before). */
+template <int WORDS, int WARPS, int KEEP, int SHARE>
 struct WsExchange {
     uint32_t words[WORDS][32];
     int lock;          /* 1 while a warp uses the exchange; only ever tried */
     int count;         /* packets in it */
+    int alive;         /* warps that have not left */
     int idle[WARPS];   /* idle lanes of the warps that have found the queue empty */
 };
 
 /* To be followed by a block barrier. */
-template <int WORDS, int WARPS>
-static __device__ __forceinline__ void ws_init(WsExchange<WORDS, WARPS> &e) {
+template <int WORDS, int WARPS, int KEEP, int SHARE>
+static __device__ __forceinline__ void ws_init(WsExchange<WORDS, WARPS, KEEP, SHARE> &e) {
     if (threadIdx.x < WARPS) e.idle[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         e.lock = 0;
         e.count = 0;
+        e.alive = (int)(blockDim.x >> 5);
     }
 }
 
 /* A warp that leaves without its packets (deadline, abort). */
-template <int WORDS, int WARPS>
-static __device__ __forceinline__ void ws_leave(WsExchange<WORDS, WARPS> &e) {
+template <int WORDS, int WARPS, int KEEP, int SHARE>
+static __device__ __forceinline__ void ws_leave(WsExchange<WORDS, WARPS, KEEP, SHARE> &e) {
     if ((threadIdx.x & 31u) == 0) *(volatile int *)&e.idle[threadIdx.x >> 5] = 0;
 }
 
@@ -74,9 +82,11 @@ static __device__ __forceinline__ void ws_leave(WsExchange<WORDS, WARPS> &e) {
    there are none and the block's other warps have idle lanes for all of this
    warp's packets, leaves them there.  Idle lanes only grow by then, apart
    from what is taken here under the lock, so packets left are taken at the
-   other warps' next try.  False: the warp has no packets and ends. */
-template <int WORDS, int WARPS, class Visit>
-static __device__ __forceinline__ bool ws_share(WsExchange<WORDS, WARPS> &e, bool &active, const Visit &visit) {
+   other warps' next try.  The last KEEP warps of a block keep what they
+   have: a few warps on an SM do not yet slow one another, and fuller ones
+   diverge more.  False: the warp has no packets and ends. */
+template <int WORDS, int WARPS, int KEEP, int SHARE, class Visit>
+static __device__ __forceinline__ bool ws_share(WsExchange<WORDS, WARPS, KEEP, SHARE> &e, bool &active, const Visit &visit) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
     const uint32_t mask = __ballot_sync(WS_FULL, active);
@@ -108,7 +118,8 @@ static __device__ __forceinline__ bool ws_share(WsExchange<WORDS, WARPS> &e, boo
     } else {
         int room = (lane < WARPS && lane != warp) ? *(volatile int *)&e.idle[lane] : 0;
         room = __reduce_add_sync(WS_FULL, room);
-        if (n <= room) {
+        const int alive = *(volatile int *)&e.alive;
+        if (n == 0 || (n <= room && alive > KEEP)) {
             if (active) {
                 WsSave save{&e.words[0][__popc(mask & below)]};
                 visit(save);
@@ -118,6 +129,7 @@ static __device__ __forceinline__ bool ws_share(WsExchange<WORDS, WARPS> &e, boo
             if (lane == 0) {
                 *(volatile int *)&e.count = n;
                 *(volatile int *)&e.idle[warp] = 0;
+                *(volatile int *)&e.alive = alive - 1;
             }
             stay = false;
         }
@@ -128,19 +140,28 @@ static __device__ __forceinline__ bool ws_share(WsExchange<WORDS, WARPS> &e, boo
     return stay;
 }
 
-/* The next packets for a warp with `need` idle lanes: [first, first + take).
-   With a fixed item size, that many.  Else a quarter of an even share of the
-   packets left at the warp's last visit, at most 128 (one visit per 128
-   packets in long runs) and at least the idle lanes: short runs fill warps
-   instead of spreading single packets over all of them, and the last packets
-   of a run go out one lane at a time. */
+/* Whether this lane takes packets: in runs too short to fill one in SHARE
+   warps of the grid, only an even share of a warp's lanes do. */
+template <int WORDS, int WARPS, int KEEP, int SHARE>
+static __device__ __forceinline__ bool ws_takes(const WsExchange<WORDS, WARPS, KEEP, SHARE> &, uint64_t N,
+                                                uint32_t fixed, uint32_t warps) {
+    return fixed != 0 || (threadIdx.x & 31u) <= N / (warps / (uint32_t)SHARE + 1u);
+}
+
+/* The next packets for a warp with `need` idle lanes: [first, end).  With a
+   fixed item size, that many.  Else a quarter of an even share of the
+   packets left at the warp's last visit, at most `most` (few visits in long
+   runs) and at least the idle lanes: short runs fill warps instead of
+   spreading single packets over all of them, and the last packets of a run
+   go out one lane at a time. */
 static __device__ __forceinline__ void ws_fetch(unsigned long long *queue, uint64_t N, uint32_t fixed,
-                                                uint32_t warps, int need, uint64_t &first, uint64_t &end) {
+                                                uint32_t most, uint32_t warps, int need, uint64_t &first,
+                                                uint64_t &end) {
     const uint64_t left = first < N ? N - first : 0;
     uint64_t take = fixed;
     if (fixed == 0) {
         take = left / ((uint64_t)warps * 4u);
-        take = take > 128 ? 128 : take;
+        take = take > most ? most : take;
         take = take < (uint64_t)need ? (uint64_t)need : take;
     }
     unsigned long long at = 0;
