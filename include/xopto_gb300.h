@@ -575,7 +575,7 @@ typedef struct McgbBatchSim {
 
 typedef struct McgbBatchConfig {
     uint32_t num_sims;
-    uint32_t packets_per_item;          /* work item size, multiple of 32    */
+    uint32_t packets_per_item;          /* largest work item, at least 32    */
     uint32_t block_size;                /* threads per block (multiple of 32)*/
     uint32_t blocks_per_sm;             /* 0 = as many as fit                */
     uint32_t num_bins;                  /* radial bins per simulation        */

@@ -100,7 +100,7 @@ class BatchedMc:
         c = _abi.McgbBatchConfig()
         c.num_sims = self._num
         c.packets_per_item = int(packets_per_item or self._packets_per_item or 256)
-        c.block_size = int(block_size or self._block_size or 128)
+        c.block_size = int(block_size or self._block_size or 256)
         c.blocks_per_sm = int(self._blocks_per_sm if blocks_per_sm is None else blocks_per_sm)
         c.num_bins = self._raxis.n
         c.math = _abi.MATH_FAST if self._fast else _abi.MATH_EXACT

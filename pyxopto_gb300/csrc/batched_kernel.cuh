@@ -29,7 +29,8 @@ namespace MCGB_NS {
 struct __align__(16) BatchPrep {
     MlLayer L[3];
     float reflectance;      /* specular reflectance of the Line source */
-    float pad[3];
+    uint32_t sim;           /* the simulation: tables are in the order of batch_prep_kernel */
+    float pad[2];
 };
 static_assert(sizeof(BatchPrep) <= MCGB_BATCH_PREP_BYTES,
               "a per-simulation table must fit the scratch record of batch_launch.h");
@@ -41,35 +42,47 @@ static __device__ __forceinline__ double cc_d(double n1, double n2) {
     return n1 > n2 ? sqrt(1.0 - (n2 / n1) * (n2 / n1)) : 0.0;
 }
 
-/* One block: packet prefix sums and the per-simulation layer tables. */
-__global__ void batch_prep_kernel(const McgbBatchSim *sims, uint32_t S, uint64_t *prefix,
-                                  BatchPrep *prep, unsigned long long *queue) {
-    __shared__ uint64_t part[1024];
-    const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    const uint32_t per = (S + nt - 1) / nt;
-    const uint32_t lo = tid * per, hi = min(S, lo + per);
-    uint64_t sum = 0;
-    for (uint32_t s = lo; s < hi; ++s) sum += sims[s].num_packets;
-    part[tid] = sum;
+/* Bucket of a simulation by the most steps that its packets can live: a
+   weight reaches the lottery after ln(1e4)/a steps of absorbed fraction a.
+   Quarter octaves of 1/a, the longest first. */
+constexpr int BATCH_BUCKETS = 128;
+static __device__ __forceinline__ int batch_bucket(const McgbBatchSim &m) {
+    float a = m.mua / (m.mua + m.mus);
+    int life = cvt_int(fminf(-4.0f * __log2f(fmaxf(a, 1e-12f)), 126.0f));
+    return BATCH_BUCKETS - 1 - clip_i(life, 0, BATCH_BUCKETS - 1);
+}
+
+/* One block: the simulations' order, packet prefix sums and the layer tables
+   in that order.  The queue hands out the longest-lived packets first: taken
+   in the caller's order, the last of them began when the rest was done, and
+   the run waited for their 1e5 serial steps alone. */
+__global__ void __launch_bounds__(1024)
+batch_prep_kernel(const McgbBatchSim *sims, uint32_t S, uint64_t *prefix, BatchPrep *prep,
+                  unsigned long long *queue) {
+    __shared__ uint32_t start[BATCH_BUCKETS];
+    __shared__ uint64_t part[32];
+    const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
+    if (tid < BATCH_BUCKETS) start[tid] = 0;
     __syncthreads();
-    if (tid == 0) {
-        uint64_t run = 0;
-        for (uint32_t i = 0; i < nt; ++i) {
-            uint64_t v = part[i];
-            part[i] = run;
-            run += v;
+    for (uint32_t s = tid; s < S; s += nt) atomicAdd(&start[batch_bucket(sims[s])], 1u);
+    __syncthreads();
+    if (tid < 32) {
+        uint32_t run = 0;
+        for (int b = 0; b < BATCH_BUCKETS; b += 32) {
+            uint32_t v = start[b + lane], sum = v;
+            for (int d = 1; d < 32; d <<= 1) {
+                uint32_t u = __shfl_up_sync(0xffffffffu, sum, d);
+                if (lane >= d) sum += u;
+            }
+            start[b + lane] = run + sum - v;
+            run += __shfl_sync(0xffffffffu, sum, 31);
         }
-        prefix[S] = run;
-        *queue = 0ull;
     }
     __syncthreads();
-    uint64_t run = part[tid];
-    for (uint32_t s = lo; s < hi; ++s) {
-        prefix[s] = run;
-        run += sims[s].num_packets;
-    }
     for (uint32_t s = tid; s < S; s += nt) {
         const McgbBatchSim m = sims[s];
+        const uint32_t at = atomicAdd(&start[batch_bucket(m)], 1u);
+        prefix[at] = m.num_packets;
         double mua = m.mua, mus = m.mus;
         double mut = mua + mus;
         float inv_mut = mut > 0.0 ? (float)(1.0 / mut) : __int_as_float(0x7f800000);
@@ -86,59 +99,186 @@ __global__ void batch_prep_kernel(const McgbBatchSim *sims, uint32_t S, uint64_t
         p.L[1].g1 = make_float4(m.n, m.mua, m.mus, (float)cc_d(m.n, m.n_above));
         p.L[1].g2 = make_float4((float)cc_d(m.n, m.n_below), 0.0f, 0.0f, 0.0f);
         pf_prepare(MCGB_PF_HG, hg1, p.L[1].pf0, p.L[1].pf1);
+#if MCGB_FAST_MATH
+        /* the square inside the multiply-add, whatever the code around */
+        p.L[1].pf0.y = __fmaf_rn(-m.g, m.g, 1.0f);
+        p.L[1].pf0.z = __fmaf_rn(m.g, m.g, 1.0f);
+#endif
         p.L[2].g0 = make_float4(m.thickness, inf, step_factor(inf), 1.0f);
         p.L[2].g1 = make_float4(m.n_below, 0.0f, 0.0f, (float)cc_d(m.n_below, m.n));
         p.L[2].g2 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         pf_prepare(MCGB_PF_HG, hg0, p.L[2].pf0, p.L[2].pf1);
         double r = ((double)m.n_above - m.n) / ((double)m.n_above + m.n);
         p.reflectance = (float)(r * r);
-        p.pad[0] = p.pad[1] = p.pad[2] = 0.0f;
-        prep[s] = p;
+        p.sim = s;
+        p.pad[0] = p.pad[1] = 0.0f;
+        prep[at] = p;
+    }
+    __syncthreads();
+    /* exclusive sums of the packet counts, one tile of the block at a time */
+    uint64_t base = 0;
+    for (uint32_t t = 0; t < S; t += nt) {
+        const uint64_t v = t + tid < S ? prefix[t + tid] : 0ull;
+        uint64_t sum = v;
+        for (int d = 1; d < 32; d <<= 1) {
+            uint64_t u = __shfl_up_sync(0xffffffffu, sum, d);
+            if ((int)lane >= d) sum += u;
+        }
+        if (lane == 31) part[tid >> 5] = sum;
+        __syncthreads();
+        uint64_t before = 0, all = 0;
+        for (uint32_t k = 0; k < nt / 32; ++k) {
+            if (k < (tid >> 5)) before += part[k];
+            all += part[k];
+        }
+        if (t + tid < S) prefix[t + tid] = base + before + sum - v;
+        base += all;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        prefix[S] = base;
+        *queue = 0ull;
     }
 }
 
-#define MCGB_FULL 0xffffffffu
+/* A packet of the batch: always in the sample layer between steps. */
+struct BatchPacket {
+    f3 pos, dir;
+    float w;
+    uint32_t rec;   /* its simulation's table */
+};
+
+/* The sample layer's constants of a lane's simulation, kept in registers:
+   one load per packet instead of three per step. */
+struct BatchLayer {
+    float factor, thickness, absorb;
+    float4 pf0;
+    float2 pf1;
+    __device__ __forceinline__ void load(const BatchPrep &p) {
+        const float4 g0 = p.L[1].g0, q = p.L[1].pf1;
+        factor = g0.z;
+        thickness = g0.y;
+        absorb = g0.w;
+        pf0 = p.L[1].pf0;
+        pf1 = make_float2(q.x, q.y);
+    }
+};
+
+typedef WsExchange<11, 8, 1, 8> BatchExchange;
+
+template <class IO>
+static __device__ __forceinline__ void batch_state(IO &io, BatchPacket &s, Rng &rng) {
+    io(s.pos.x); io(s.pos.y); io(s.pos.z);
+    io(s.dir.x); io(s.dir.y); io(s.dir.z);
+    io(s.w); io(s.rec);
+    io(rng.x); io(rng.a);
+}
+
+/* One step, as mcml_step_weight: the scattered direction is computed before
+   it is known whether the path stays in the layer.  True when the packet
+   ended.  What bounds a batch is issue, and for its longest packets (1e5
+   steps) the latency of a step: with the layer's constants in registers, one
+   block of code per step, the longest-lived simulations first and merged
+   last packets, 200 simulations of the benchmark's range took 180 ms
+   instead of 268, 32 smaller ones 101 instead of 138. */
+template <bool RMAX>
+static __device__ __forceinline__ bool batch_step(const McgbBatchConfig &cfg, const BatchPrep *prep,
+                                                  const BatchLayer &c, BatchPacket &s, Rng &rng,
+                                                  float rmax2, uint64_t *tally) {
+    const float u = rng.next();
+    Rng srng = rng;
+    f3 sdir = s.dir;
+    float az, ct = pf_sample<MCGB_PF_HG>(c.pf0, make_float4(c.pf1.x, c.pf1.y, 0.0f, 0.0f), nullptr, srng,
+                                         &az, sdir);
+    scatter_direction<true>(sdir, ct, az);
+    float step = sample_step(u, c.factor);
+    step = fminf(step, FLT_MAX);
+    const float z = s.pos.z + step * s.dir.z;
+    bool done = false;
+    int layer = 1, next = 1;
+    if (z < 0.0f || z >= c.thickness) {
+        if (z < 0.0f) {
+            --next;
+            if (fabsf(s.dir.z) != 0.0f) step = mc_div(0.0f - s.pos.z, s.dir.z);
+        }
+        if (s.pos.z + step * s.dir.z >= c.thickness) {
+            ++next;
+            if (fabsf(s.dir.z) != 0.0f) step = mc_div(c.thickness - s.pos.z, s.dir.z);
+        }
+        s.pos.x = s.pos.x + s.dir.x * step;
+        s.pos.y = s.pos.y + s.dir.y * step;
+        s.pos.z = s.pos.z + s.dir.z * step;
+        if (next > 1) s.pos.z = c.thickness;
+        if (next < 1) s.pos.z = 0.0f;
+        if (next != 1) {
+            const BatchPrep &p = prep[s.rec];
+            mcml_boundary(p.L, layer, next, s.dir, rng);
+            if (layer != 1) {
+                if (layer == 0) {
+                    /* Radial detector, xopto/mcml/mcdetector/radial.py:117-150 */
+                    float r = mc_sqrt(s.pos.x * s.pos.x + s.pos.y * s.pos.y);
+                    int idx = clip_i(cvt_int(r * cfg.inv_dr), 0, (int)cfg.num_bins - 1);
+                    uint32_t wi = weight_to_u32(s.w, 1.0f);
+                    if (wi > 0) accu_add(tally, (uint64_t)p.sim * cfg.num_bins + idx, wi);
+                }
+                done = true;
+            }
+        }
+    } else {
+        s.pos.x = s.pos.x + s.dir.x * step;
+        s.pos.y = s.pos.y + s.dir.y * step;
+        s.pos.z = s.pos.z + s.dir.z * step;
+    }
+    if (next == 1) {
+        float deposit = s.w * c.absorb;
+        s.w -= deposit;
+        rng = srng;
+        s.dir = sdir;
+        if (s.w < 1e-4f) {
+            if (rng.next() > 0.1f) done = true;
+            else s.w = mc_div(s.w, 0.1f);
+        }
+    }
+    if (RMAX && dot3(s.pos, s.pos) > rmax2) done = true;
+    return done;
+}
 
 template <bool RMAX>
 __global__ void __launch_bounds__(256)
 batched_kernel(const McgbBatchConfig cfg, const uint32_t *__restrict__ mult,
                const uint64_t *__restrict__ prefix, const BatchPrep *__restrict__ prep,
                unsigned long long *queue, uint64_t *tally, uint64_t *counters, uint64_t deadline_ns) {
+    __shared__ BatchExchange share;
+    ws_init(share);
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t S = cfg.num_sims;
     const uint64_t total = prefix[S];
-    const uint64_t B = cfg.packets_per_item;
-    const float inv_dr = cfg.inv_dr;
-    const int last_bin = (int)cfg.num_bins - 1;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const bool takes = ws_takes(share, total, 0u, warps);
     const float rmax2 = cfg.rmax * cfg.rmax;
     const uint64_t t_deadline = globaltimer_ns() + deadline_ns;
 
     uint64_t item_next = 0, item_end = 0;   /* warp-uniform */
     bool more = true;                         /* warp-uniform */
     bool active = false;
-    f3 pos{0.0f, 0.0f, 0.0f}, dir{0.0f, 0.0f, 1.0f};
-    float w = 0.0f;
-    int layer = 1;
-    uint32_t sim = 0;
+    BatchPacket s;
+    s.rec = 0;
+    BatchLayer c;
     Rng rng{0ull, 0u};
-    const MlLayer *L = prep[0].L;
     uint64_t steps = 0, packets = 0;
     uint32_t iter = 0, status = 0;
 
     for (;;) {
         /* refill idle lanes with the next packets of the warp's item */
-        uint32_t need = __ballot_sync(MCGB_FULL, !active);
+        uint32_t need = __ballot_sync(WS_FULL, takes && !active);
         while (need && more) {
             if (item_next >= item_end) {
-                unsigned long long item = 0;
-                if (lane == 0) item = atomicAdd(queue, 1ull);
-                item = __shfl_sync(MCGB_FULL, item, 0);
-                item_next = (uint64_t)item * B;
+                ws_fetch(queue, total, 0u, cfg.packets_per_item, warps, __popc(need), item_next, item_end);
                 if (item_next >= total) {
                     more = false;
                     break;
                 }
-                item_end = min(item_next + B, total);
             }
             uint32_t avail = (uint32_t)min(item_end - item_next, (uint64_t)32);
             uint32_t rank = __popc(need & ((1u << lane) - 1u));
@@ -152,80 +292,45 @@ batched_kernel(const McgbBatchConfig cfg, const uint32_t *__restrict__ mult,
                     if (prefix[mid] <= g) lo = mid;
                     else hi = mid - 1u;
                 }
-                sim = lo;
+                s.rec = lo;
+                const BatchPrep &p = prep[lo];
                 uint64_t x;
                 uint32_t a;
-                br_packet_stream(cfg.seed, sim, g - prefix[sim], mult, cfg.num_multipliers, &x, &a);
+                br_packet_stream(cfg.seed, p.sim, g - prefix[lo], mult, cfg.num_multipliers, &x, &a);
                 rng = Rng{x, a};
-                L = prep[sim].L;
+                c.load(p);
                 /* Line source at normal incidence (xopto/mcml/mcsource/line.py:95-108) */
-                w = 1.0f - prep[sim].reflectance;
-                pos = f3{0.0f, 0.0f, 0.0f};
-                dir = f3{0.0f, 0.0f, 1.0f};
-                layer = 1;
+                s.w = 1.0f - p.reflectance;
+                s.pos = f3{0.0f, 0.0f, 0.0f};
+                s.dir = f3{0.0f, 0.0f, 1.0f};
                 active = true;
             }
-            uint32_t taken = __ballot_sync(MCGB_FULL, mine);
+            uint32_t taken = __ballot_sync(WS_FULL, mine);
             item_next += __popc(taken);
             need &= ~taken;
         }
-        if (!__any_sync(MCGB_FULL, active)) break;
+        if (!more) {
+            const bool had = active;
+            if (!ws_share(share, active, [&](auto &io) { batch_state(io, s, rng); })) break;
+            if (active && !had) c.load(prep[s.rec]);
+        }
 
         /* sixteen steps between refills, two step bodies per loop
            iteration: the refill's ballots and queue reads cost more than the
            idle lanes of a packet that ends early (+2.4 % against eight steps
            without unrolling) */
+        uint32_t taken = 0;
 #pragma unroll 2
         for (int k = 0; k < 16; ++k) {
             if (active) {
-                const float4 g0 = L[layer].g0;
-                ++steps;
-                float step = sample_step(rng.next(), g0.z);
-                step = fminf(step, FLT_MAX);
-                int next = layer;
-                if (pos.z + step * dir.z < g0.x) {
-                    --next;
-                    if (fabsf(dir.z) != 0.0f) step = mc_div(g0.x - pos.z, dir.z);
-                }
-                if (pos.z + step * dir.z >= g0.y) {
-                    ++next;
-                    if (fabsf(dir.z) != 0.0f) step = mc_div(g0.y - pos.z, dir.z);
-                }
-                pos.x = pos.x + dir.x * step;
-                pos.y = pos.y + dir.y * step;
-                pos.z = pos.z + dir.z * step;
-                if (layer < next) pos.z = g0.y;
-                if (layer > next) pos.z = g0.x;
-                bool done = false;
-                if (next != layer) {
-                    mcml_boundary(L, layer, next, dir, rng);
-                    if (!(layer > 0 && layer < 2)) {
-                        if (layer <= 0) {
-                            /* Radial detector, xopto/mcml/mcdetector/radial.py:117-150 */
-                            float r = mc_sqrt(pos.x * pos.x + pos.y * pos.y);
-                            int idx = clip_i(cvt_int(r * inv_dr), 0, last_bin);
-                            uint32_t wi = weight_to_u32(w, 1.0f);
-                            if (wi > 0) accu_add(tally, (uint64_t)sim * cfg.num_bins + idx, wi);
-                        }
-                        done = true;
-                    }
-                } else {
-                    float deposit = w * g0.w;
-                    w -= deposit;
-                    float az, ct = pf_sample<MCGB_PF_HG>(L[layer].pf0, L[layer].pf1, nullptr, rng, &az, dir);
-                    scatter_direction(dir, ct, az);
-                    if (w < 1e-4f) {
-                        if (rng.next() > 0.1f) done = true;
-                        else w = mc_div(w, 0.1f);
-                    }
-                }
-                if (RMAX && dot3(pos, pos) > rmax2) done = true;
-                if (done) {
+                ++taken;
+                if (batch_step<RMAX>(cfg, prep, c, s, rng, rmax2, tally)) {
                     active = false;
                     ++packets;
                 }
             }
         }
+        steps += taken;
         iter += 16;
         if ((iter & 1023u) == 0) {
             uint32_t stop = 0;
@@ -233,18 +338,15 @@ batched_kernel(const McgbBatchConfig cfg, const uint32_t *__restrict__ mult,
                 if (globaltimer_ns() > t_deadline) stop = MCGB_STATUS_TIMEOUT;
                 else if (*(volatile uint64_t *)(counters + MCGB_CNT_ABORT)) stop = MCGB_STATUS_ABORTED;
             }
-            stop = __shfl_sync(MCGB_FULL, stop, 0);
+            stop = __shfl_sync(WS_FULL, stop, 0);
             if (stop) {
                 status |= stop;
+                ws_leave(share);
                 break;
             }
         }
     }
-    atomicAdd((unsigned long long *)(counters + MCGB_CNT_STEPS), (unsigned long long)steps);
-    atomicAdd((unsigned long long *)(counters + MCGB_CNT_PACKETS), (unsigned long long)packets);
-    if (lane == 0) atomicAdd((unsigned long long *)(counters + MCGB_CNT_THREADS), 32ull);
-    if (status && lane == 0)
-        atomicOr((unsigned long long *)(counters + MCGB_CNT_STATUS), (unsigned long long)status);
+    warp_finish(counters, steps, packets, status);
 }
 
 }  // namespace MCGB_NS
