@@ -708,6 +708,35 @@ typedef struct McgbAdamwTensor {
 int mcgb_mlp_adamw_multi(const McgbAdamwTensor *tensors, int count, float lr, float beta1, float beta2,
                          float eps, int step, void *stream);
 
+/* One whole training step of an MLP with GELU hidden layers and a 32-column
+   linear output: forward pass, loss gradient (mcgb_mlp_loss_grad), backward
+   pass, tied input columns (mcgb_mlp_tie_columns, tie_count = 0: none) and
+   AdamW.  tensors[2 i] holds layer i's weights [rows = outputs, cols =
+   inputs] with both bf16 copies, tensors[2 i + 1] its bias [1, outputs];
+   their grad arrays receive the gradients.  h[i] and pre[i] receive layer
+   i's output and pre-activation, dpre[i] the gradient of the latter; loss
+   [ceil(m / 256)] the loss of every 256 rows.  x [m, cols of layer 0] bf16
+   and target [m, 32] are 16-byte aligned, scratch holds
+   mcgb_mlp_train_scratch(tensors, layers, m) floats.  tcgen05 path only. */
+typedef struct McgbMlpStep {
+    const McgbAdamwTensor *tensors;                 /* host array, 2 * layers */
+    const uint16_t *x;
+    uint16_t *x_copy;                               /* receives x, or NULL    */
+    const float *target;
+    const float *loss_weights;                      /* [32] or NULL           */
+    float *loss;
+    float *scratch;
+    uint16_t *h[MCGB_ADAMW_MAX_TENSORS / 2];
+    float *pre[MCGB_ADAMW_MAX_TENSORS / 2];
+    uint16_t *dpre[MCGB_ADAMW_MAX_TENSORS / 2];
+    int32_t layers, m, nv, mode;
+    int32_t tie_count, tie_shift, step, reserved;
+    float scale, lr, beta1, beta2, eps, reserved2;
+} McgbMlpStep;
+
+int mcgb_mlp_train_step(const McgbMlpStep *step, void *stream);
+uint64_t mcgb_mlp_train_scratch(const McgbAdamwTensor *tensors, int layers, int m);
+
 /* GEMM implementation behind the mcgb_mlp_* calls: 0 = tcgen05.mma on
    128 x 64 tiles with the FP32 accumulator in tensor memory (the default),
    1 = the warp-level mma.sync kernel on 64 x 64 tiles.  path = -1 only

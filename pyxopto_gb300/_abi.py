@@ -159,10 +159,22 @@ class McgbAdamwTensor(C.Structure):
 
 ADAMW_MAX_TENSORS = 16
 
+
+class McgbMlpStep(C.Structure):
+    _fields_ = [('tensors', C.POINTER(McgbAdamwTensor)), ('x', C.c_void_p), ('x_copy', C.c_void_p),
+                ('target', C.c_void_p),
+                ('loss_weights', C.c_void_p), ('loss', C.c_void_p), ('scratch', C.c_void_p),
+                ('h', C.c_void_p * (ADAMW_MAX_TENSORS // 2)), ('pre', C.c_void_p * (ADAMW_MAX_TENSORS // 2)),
+                ('dpre', C.c_void_p * (ADAMW_MAX_TENSORS // 2)),
+                ('layers', i32), ('m', i32), ('nv', i32), ('mode', i32),
+                ('tie_count', i32), ('tie_shift', i32), ('step', i32), ('reserved', i32),
+                ('scale', f32), ('lr', f32), ('beta1', f32), ('beta2', f32), ('eps', f32), ('reserved2', f32)]
+
+
 SIZEOF_KINDS = [McgbLayer, McgbSource, McgbDetector, McgbFluence, McgbTrace,
                 McgbMaterial, McgbMcmlConfig, McgbMcvoxConfig, McgbBuffers,
                 McgbRunOptions, McgbPf, McgbBatchSim, McgbBatchConfig, McgbSurface,
-                McgbSamplingVolume, McgbAdamwTensor]
+                McgbSamplingVolume, McgbAdamwTensor, McgbMlpStep]
 
 
 def check_layout(sizeof_fn):

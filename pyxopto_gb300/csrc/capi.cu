@@ -320,6 +320,7 @@ int mcgb_sizeof(int kind) {
         case 13: return (int)sizeof(McgbSurface);
         case 14: return (int)sizeof(McgbSamplingVolume);
         case 15: return (int)sizeof(McgbAdamwTensor);
+        case 16: return (int)sizeof(McgbMlpStep);
         default: return -1;
     }
 }

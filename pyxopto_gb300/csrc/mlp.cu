@@ -411,6 +411,8 @@ int launch_gemm(const bf16 *A, int lda, const bf16 *B, int ldb, int R, int Cc, i
     return check_launch(what);
 }
 
+#include "mlp_step.cuh"
+
 }  // namespace
 
 extern "C" {
@@ -545,6 +547,161 @@ int mcgb_mlp_adamw_multi(const McgbAdamwTensor *tensors, int count, float lr, fl
     if (blocks > most) blocks = most;
     adamw_multi_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(p);
     return check_launch("mlp adamw multi");
+}
+
+uint64_t mcgb_mlp_train_scratch(const McgbAdamwTensor *tensors, int layers, int m) {
+    if (!tensors || layers < 1 || layers > STEP_MAX_LAYERS || m <= 0) return 0;
+    const uint64_t groups = (uint64_t)(m + 31) / 32;
+    uint64_t n = (2 * groups + 3) / 4 * 4;
+    for (int i = 0; i < layers; ++i) {
+        int rows, parts, slices;
+        step_slices(tensors[2 * i], m, step_tiles(tensors, layers), rows, parts, slices);
+        n += (uint64_t)slices * tensors[2 * i].rows * tensors[2 * i].cols + groups * (uint64_t)tensors[2 * i].rows;
+    }
+    return n;
+}
+
+int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
+    if (!s || !s->tensors || s->layers < 2 || s->layers > STEP_MAX_LAYERS || s->step < 1 || !s->x || !s->target ||
+        !s->loss || !s->scratch || s->mode < 0 || s->mode > 1)
+        return fail(MCGB_E_INVALID, "bad train_step arguments");
+    const int L = s->layers, m = s->m;
+    const McgbAdamwTensor *t = s->tensors;
+    if (g_gemm_path != 0) return fail(MCGB_E_UNSUPPORTED, "train_step runs on the tcgen05 GEMM path only");
+    for (int i = 0; i < L; ++i) {
+        const McgbAdamwTensor &w = t[2 * i], &b = t[2 * i + 1];
+        int r = shape_ok(m, w.rows, w.cols);
+        if (r) return r;
+        if (!w.w || !w.w_bf16 || !w.wt_bf16 || !w.grad || !w.m || !w.v || !b.w || !b.w_bf16 || !b.grad || !b.m ||
+            !b.v || !s->h[i] || !s->pre[i] || !s->dpre[i] || b.rows != 1 || b.cols != w.rows ||
+            (i && w.cols != t[2 * i - 2].rows))
+            return fail(MCGB_E_INVALID, "bad train_step layer %d", i);
+    }
+    const int nout = t[2 * L - 2].rows;
+    if (nout != 32 || s->nv < 1 || s->nv > nout)
+        return fail(MCGB_E_UNSUPPORTED, "train_step takes a 32-column output layer");
+    if (s->tie_count < 0 || (s->tie_count && (s->tie_shift < s->tie_count || s->tie_count + s->tie_shift > t[0].cols)))
+        return fail(MCGB_E_INVALID, "bad tied columns");
+    const uintptr_t all = (uintptr_t)s->x | (uintptr_t)s->x_copy | (uintptr_t)s->target |
+                          (uintptr_t)s->scratch;
+    if (all & 15u) return fail(MCGB_E_INVALID, "train_step operands must be 16-byte aligned");
+
+    cudaStream_t st = (cudaStream_t)stream;
+    int rows[STEP_MAX_LAYERS], parts[STEP_MAX_LAYERS], slices[STEP_MAX_LAYERS];
+    const int groups = (m + 31) / 32;
+    float *at = s->scratch;
+    float *loss_part = at;
+    at += (2 * groups + 3) / 4 * 4;
+    StepUpdate up;
+    memset(&up, 0, sizeof(up));
+    float *dw[STEP_MAX_LAYERS], *db[STEP_MAX_LAYERS];
+    for (int i = 0; i < L; ++i) {
+        step_slices(t[2 * i], m, step_tiles(t, L), rows[i], parts[i], slices[i]);
+        dw[i] = at;
+        at += (size_t)slices[i] * t[2 * i].rows * t[2 * i].cols;
+    }
+    for (int i = 0; i < L; ++i) {
+        db[i] = at;
+        at += (size_t)groups * t[2 * i].rows;
+    }
+    const int mt = (m + TBM - 1) / TBM;
+    auto wide = [&](int cols) { return (long)mt * ((cols + 63) / 64) >= sm_count(); };
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < L && e == cudaSuccess; ++i) {
+        StepForward f;
+        memset(&f, 0, sizeof(f));
+        f.x = (const bf16 *)(i ? s->h[i - 1] : s->x);
+        f.copy = i ? nullptr : (bf16 *)s->x_copy;
+        f.w = (const bf16 *)t[2 * i].w_bf16;
+        f.bias = t[2 * i + 1].w;
+        f.h = (bf16 *)s->h[i];
+        f.pre = s->pre[i];
+        f.m = m;
+        f.n = t[2 * i].rows;
+        f.k = t[2 * i].cols;
+        f.act = i + 1 < L;
+        if (i + 1 == L) {
+            f.target = s->target;
+            f.wcol = s->loss_weights;
+            f.dpre = (bf16 *)s->dpre[i];
+            f.part = db[i];
+            f.loss_part = loss_part;
+            f.nv = s->nv;
+            f.mode = s->mode;
+            f.scale = s->scale;
+            f.clip = 4.0f;
+            e = step_launch_tc(step_forward<32, true>, TcShape<32>::SMEM, dim3(1, mt), st, f);
+        } else if (wide(f.n)) {
+            e = step_launch_tc(step_forward<64, false>, TcShape<64>::SMEM, dim3((f.n + 63) / 64, mt), st, f);
+        } else {
+            e = step_launch_tc(step_forward<32, false>, TcShape<32>::SMEM, dim3((f.n + 31) / 32, mt), st, f);
+        }
+    }
+    for (int i = L - 1; i > 0 && e == cudaSuccess; --i) {
+        StepBackward f;
+        f.dpre = (const bf16 *)s->dpre[i];
+        f.wt = (const bf16 *)t[2 * i].wt_bf16;
+        f.pre = s->pre[i - 1];
+        f.out = (bf16 *)s->dpre[i - 1];
+        f.part = db[i - 1];
+        f.m = m;
+        f.n = t[2 * i].rows;
+        f.k = t[2 * i].cols;
+        f.act = 1;
+        e = wide(f.k) ? step_launch_tc(step_backward<64>, TcShape<64>::SMEM, dim3((f.k + 63) / 64, mt), st, f)
+                      : step_launch_tc(step_backward<32>, TcShape<32>::SMEM, dim3((f.k + 31) / 32, mt), st, f);
+    }
+    if (e == cudaSuccess) {
+        StepWeights f;
+        memset(&f, 0, sizeof(f));
+        f.layers = L;
+        f.m = m;
+        int first = 0;
+        for (int i = 0; i < L; ++i) {
+            StepWeightLayer &l = f.layer[i];
+            l.dpre = (const bf16 *)s->dpre[i];
+            l.x = (const bf16 *)(i ? s->h[i - 1] : s->x);
+            l.out = dw[i];
+            l.n = t[2 * i].rows;
+            l.k = t[2 * i].cols;
+            l.first = first;
+            l.rows = rows[i];
+            l.parts = parts[i];
+            l.slices = slices[i];
+            first += slices[i] * ((l.n + TBM - 1) / TBM) * ((l.k + STEP_BN - 1) / STEP_BN);
+        }
+        e = step_launch_tc(step_weights, TcShape<STEP_BN>::SMEM, dim3(first), st, f);
+    }
+    if (e == cudaSuccess) {
+        up.a.count = 2 * L;
+        up.a.lr = s->lr;
+        up.a.b1 = s->beta1;
+        up.a.b2 = s->beta2;
+        up.a.eps = s->eps;
+        up.a.c1 = 1.0f - powf(s->beta1, (float)s->step);
+        up.a.c2 = 1.0f - powf(s->beta2, (float)s->step);
+        for (int i = 0; i < 2 * L; ++i) up.a.t[i] = t[i];
+        for (int i = 0; i < L; ++i) {
+            up.dw[i] = dw[i];
+            up.db[i] = db[i];
+            up.slices[i] = slices[i];
+            up.wstart[i + 1] = up.wstart[i] + (uint64_t)t[2 * i].rows * (uint64_t)t[2 * i].cols;
+            up.bstart[i + 1] = up.bstart[i] + (t[2 * i].rows + 31) / 32;
+        }
+        up.weights = up.wstart[L];
+        up.layers = L;
+        up.groups = groups;
+        up.tie_count = s->tie_count;
+        up.tie_shift = s->tie_shift;
+        up.loss_part = loss_part;
+        up.loss = s->loss;
+        up.m = m;
+        up.weight_blocks = (int)((up.weights + 255) / 256);
+        up.bias_blocks = up.bstart[L];
+        e = step_launch(step_update, dim3(up.weight_blocks + up.bias_blocks + 1), 256, 0, st, up);
+    }
+    if (e != cudaSuccess) return fail(MCGB_E_CUDA, "mlp train step: %s", cudaGetErrorString(e));
+    return MCGB_OK;
 }
 
 }  // extern "C"

@@ -4,7 +4,7 @@
  * anonymous namespace, after the bf16 typedef, gelu() and the EPI_* codes.
  *
  * C[R, Cc] = sum_l A(r, l) B(c, l) over the reduction range of blockIdx.z's
- * slice, one CTA of 128 threads per 128 x BN output tile (BN = 64 or 32):
+ * slice, one CTA of 256 threads per 128 x BN output tile (BN = 64 or 32):
  * the M = 128, N = BN shape of tcgen05.mma.cta_group::1.kind::f16 with BF16
  * operands and an FP32 accumulator of BN TMEM columns.
  *
@@ -27,7 +27,8 @@
  * four later.
  *
  * Epilogue: tcgen05.ld of 32 lanes x 16 columns per warp (warp w owns TMEM
- * lanes 32w..32w+31, one output row per thread), then the same fused
+ * lanes 32 (w mod 4).., one output row per thread; warps 0-3 take the even
+ * groups of 16 columns, warps 4-7 the odd ones), then the same fused
  * epilogues as the mma.sync kernel, stored 16 columns per thread.
  *
  * Every wait is bounded by the global timer (one second); a CTA that gives
@@ -35,7 +36,7 @@
  */
 #pragma once
 
-constexpr int TBM = 128, TBK = 64, TNT = 128;
+constexpr int TBM = 128, TBK = 64, TNT = 256;
 constexpr uint32_t TC_A_BYTES = TBM * TBK * 2;                 /* 16 KB */
 constexpr uint64_t TC_WAIT_NS = 1000000000ull;
 
@@ -156,7 +157,7 @@ __device__ __forceinline__ void tc_cp_wait(int n) {
 /* Operand staging with cp.async, 16 bytes per copy, zero-filled outside the
    matrix.  X(r, l) = TR ? X[l*ld + r] : X[r*ld + l]; rows >= R and
    reduction indices >= L are zero (R, L, r0, l0 are multiples of 8).
-   Vector j of thread t is v = t + 128 j:
+   Vector j of thread t is v = t + TNT j:
      K-major (!TR): row-in-group v & 7, reduction group (v >> 3) & 7, row
        group v >> 6; 16 bytes of 8 reduction indices of one row, stored as
        row (v & 7) of core matrix (row group, reduction group);
@@ -194,20 +195,29 @@ struct TcStage {
     }
 };
 
-template <int BN, bool TA, bool TB, int EPI>
-__global__ void __launch_bounds__(TNT)
-gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb, int R, int Cc, int L,
-        int l_slice, const float *__restrict__ bias, int act, bf16 *Cb, float *Cf, float *pre, int ldc) {
+/* Waits for the kernels before this one in the stream and lets the next one
+   start its set-up; both do nothing in a launch without programmatic
+   serialization. */
+__device__ __forceinline__ void tc_after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+/* The product of one output tile: rows r0.. of op(A) and c0.. of op(B) over
+   the reduction range [lb, le).  Returns with the accumulator rows 32 (w mod
+   4).. of warp w in those TMEM lanes of `tmem`, and false when a wait ran
+   out.  The reduction starts a new accumulator, BN columns on, every `part`
+   chunks (COLS / BN of them at most). */
+template <int BN, bool TA, bool TB, int COLS = BN>
+__device__ __forceinline__ bool tc_product(uint8_t *tc_smem, const bf16 *__restrict__ A, int lda,
+                                           const bf16 *__restrict__ B, int ldb, int R, int Cc, int r0, int c0,
+                                           int lb, int le, uint32_t &tmem, int part = 1 << 30) {
     typedef TcShape<BN> Sh;
     typedef TcStage<TA, TBM> StA;
     typedef TcStage<TB, BN> StB;
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(tc_smem);
     const uint32_t bar0 = sbase + Sh::BARS, taddr_slot = sbase + Sh::TADDR;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r0 = blockIdx.y * TBM, c0 = blockIdx.x * BN;
-    const int lb = blockIdx.z * l_slice;
-    const int le = min(L, lb + l_slice);
+    const int tid = threadIdx.x, warp = tid >> 5;
     const int nch = le > lb ? (le - lb + TBK - 1) / TBK : 0;
 
     if (tid == 0) {
@@ -217,10 +227,11 @@ gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(taddr_slot),
-                     "r"((uint32_t)BN)
+                     "r"((uint32_t)COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    tc_after_previous();
     /* the first TC_STAGES chunks go in flight at once */
     for (int i = 0; i < nch && i < TC_STAGES; ++i) {
         const uint32_t st = sbase + i * Sh::STAGE;
@@ -231,7 +242,7 @@ gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tc_smem + Sh::TADDR);
+    tmem = *reinterpret_cast<volatile uint32_t *>(tc_smem + Sh::TADDR);
     const uint64_t t_end = tc_clock_ns() + TC_WAIT_NS;
 
     bool ok = true;
@@ -247,8 +258,8 @@ gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb
             const uint32_t a = sbase + s * Sh::STAGE, b = a + TC_A_BYTES;
 #pragma unroll
             for (int kk = 0; kk < TBK / 16; ++kk)
-                tc_mma(tmem, tc_desc(a + 256u * kk), tc_desc(b + 256u * kk), tc_idesc<BN, TA, TB>(),
-                       (i | kk) ? 1u : 0u);
+                tc_mma(tmem + (uint32_t)(i / part * BN), tc_desc(a + 256u * kk), tc_desc(b + 256u * kk),
+                       tc_idesc<BN, TA, TB>(), (i % part | kk) ? 1u : 0u);
             tc_commit(bar);
         }
         if (i + TC_STAGES < nch) {
@@ -266,22 +277,83 @@ gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb
         ok = tc_mbar_wait(bar0 + 8 * (i % TC_STAGES), (uint32_t)(i / TC_STAGES) & 1u, t_end);
     }
     tc_fence_after();
+    return ok;
+}
 
-    const int r = r0 + warp * 32 + lane;
+/* Columns 16 j .. of the tile: this thread's row, zero without a reduction
+   and NaN after a wait that ran out. */
+__device__ __forceinline__ void tc_row16(uint32_t tmem, int j, bool any, bool ok, float (&v)[16]) {
+    if (any) {
+        tc_ld16(tmem + ((threadIdx.x & 96u) << 16) + (uint32_t)(j * 16), v);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+    }
+    if (!ok) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = __int_as_float(0x7fc00000);
+    }
+}
+
+template <int COLS>
+__device__ __forceinline__ void tc_release(uint32_t tmem) {
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)COLS)
+                     : "memory");
+}
+
+/* The tile row of this thread. */
+__device__ __forceinline__ int tc_row() { return (int)(threadIdx.x & 127u); }
+
+__device__ __forceinline__ void tc_store16(float *p, const float (&v)[16]) {
+    float4 *p4 = reinterpret_cast<float4 *>(p);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) p4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+
+__device__ __forceinline__ void tc_load16(const float *p, float (&v)[16]) {
+    const float4 *p4 = reinterpret_cast<const float4 *>(p);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 f = p4[q];
+        v[4 * q] = f.x;
+        v[4 * q + 1] = f.y;
+        v[4 * q + 2] = f.z;
+        v[4 * q + 3] = f.w;
+    }
+}
+
+__device__ __forceinline__ void tc_store16(bf16 *p, const float (&v)[16]) {
+    uint32_t h[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        __nv_bfloat162 t2 = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+        h[q] = *reinterpret_cast<uint32_t *>(&t2);
+    }
+    uint4 *c4 = reinterpret_cast<uint4 *>(p);
+    c4[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    c4[1] = make_uint4(h[4], h[5], h[6], h[7]);
+}
+
+template <int BN, bool TA, bool TB, int EPI>
+__global__ void __launch_bounds__(TNT)
+gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb, int R, int Cc, int L,
+        int l_slice, const float *__restrict__ bias, int act, bf16 *Cb, float *Cf, float *pre, int ldc) {
+    extern __shared__ __align__(1024) uint8_t tc_smem[];
+    const int r0 = blockIdx.y * TBM, c0 = blockIdx.x * BN;
+    const int lb = blockIdx.z * l_slice;
+    const int le = min(L, lb + l_slice);
+    uint32_t tmem;
+    const bool ok = tc_product<BN, TA, TB>(tc_smem, A, lda, B, ldb, R, Cc, r0, c0, lb, le, tmem);
+
+    const int r = r0 + tc_row();
 #pragma unroll 1
-    for (int j = 0; j < BN / 16; ++j) {
+    for (int j = threadIdx.x >> 7; j < BN / 16; j += TNT / 128) {
         const int c = c0 + j * 16;
         float v[16];
-        if (nch > 0) {
-            tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * 16), v);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = 0.0f;
-        }
-        if (!ok) {
-#pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = __int_as_float(0x7fc00000);
-        }
+        tc_row16(tmem, j, le > lb, ok, v);
         if (r >= R || c >= Cc) continue;
         const size_t o = (size_t)r * ldc + c;
         if (EPI == EPI_FWD) {
@@ -289,40 +361,17 @@ gemm_tc(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb
 #pragma unroll
                 for (int q = 0; q < 16; ++q) v[q] += bias[c + q];
             }
-            if (pre) {
-                float4 *p4 = reinterpret_cast<float4 *>(pre + o);
+            if (pre) tc_store16(pre + o, v);
+            if (act) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) p4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                for (int q = 0; q < 16; ++q) v[q] = gelu(v[q]);
             }
-            uint32_t h[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float x0 = act ? gelu(v[2 * q]) : v[2 * q], x1 = act ? gelu(v[2 * q + 1]) : v[2 * q + 1];
-                __nv_bfloat162 t2 = __floats2bfloat162_rn(x0, x1);
-                h[q] = *reinterpret_cast<uint32_t *>(&t2);
-            }
-            uint4 *c4 = reinterpret_cast<uint4 *>(Cb + o);
-            c4[0] = make_uint4(h[0], h[1], h[2], h[3]);
-            c4[1] = make_uint4(h[4], h[5], h[6], h[7]);
+            tc_store16(Cb + o, v);
         } else if (EPI == EPI_BF16) {
-            uint32_t h[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                __nv_bfloat162 t2 = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-                h[q] = *reinterpret_cast<uint32_t *>(&t2);
-            }
-            uint4 *c4 = reinterpret_cast<uint4 *>(Cb + o);
-            c4[0] = make_uint4(h[0], h[1], h[2], h[3]);
-            c4[1] = make_uint4(h[4], h[5], h[6], h[7]);
+            tc_store16(Cb + o, v);
         } else {
-            float4 *p4 = reinterpret_cast<float4 *>(Cf + (size_t)blockIdx.z * R * ldc + o);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) p4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            tc_store16(Cf + (size_t)blockIdx.z * R * ldc + o, v);
         }
     }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN)
-                     : "memory");
+    tc_release<BN>(tmem);
 }

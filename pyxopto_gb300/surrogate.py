@@ -131,6 +131,7 @@ class Mlp:
         self.dw = [torch.empty_like(w) for w in self.w]
         self.db = [torch.empty_like(b) for b in self.b]
         self._adamw_tab = None          # holds the gradient pointers
+        self._step_tab = None
         nscr = 0
         for i in range(len(self.w)):
             nscr = max(nscr, int(self.lib.mcgb_mlp_bwd_weight_scratch(batch, self.pads[i + 1], self.pads[i])),
@@ -232,8 +233,48 @@ class Mlp:
                                                self._p(self.db[i]), self._p(self.mb[i]), self._p(self.vb[i]),
                                                1, n, lr, b1, b2, eps, 0.0, self.step_count, self._stream()))
 
+    def _step(self):
+        """The one-call training step's table (mcgb_mlp_train_step): every
+        pointer that stays the same until the buffers change."""
+        if self._step_tab is None:
+            s = _abi.McgbMlpStep()
+            nl = len(self.w)
+            s.tensors = self._adamw_table()
+            nscr = int(self.lib.mcgb_mlp_train_scratch(s.tensors, nl, self.batch))
+            self._step_scratch = self.torch.empty((max(nscr, 1),), dtype=self.torch.float32, device='cuda')
+            s.scratch, s.loss = self._step_scratch.data_ptr(), self.loss_part.data_ptr()
+            for i in range(nl):
+                s.h[i], s.pre[i], s.dpre[i] = (v.data_ptr() for v in (self.h[i + 1], self.pre[i], self.dpre[i]))
+            s.layers = nl
+            s.tie_count = s.tie_shift = self.sizes[0] if self.split else 0
+            s.beta1, s.beta2, s.eps = 0.9, 0.999, 1e-8
+            self._step_tab = s
+        return self._step_tab
+
+    def _one_call(self, x, t, m):
+        """Whether the fused step takes these operands."""
+        torch = self.torch
+        return (self.acts[-1] == 0 and all(self.acts[:-1]) and 2 <= len(self.w) <= _abi.ADAMW_MAX_TENSORS // 2 and
+                self.pads[-1] == 32 and self.lib.mcgb_mlp_gemm_path(-1) == 0 and
+                x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1:] == (IN_PAD,) and
+                x.data_ptr() % 16 == 0 and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and
+                t.data_ptr() % 16 == 0 and t.numel() >= m * self.pads[-1])
+
     def train_step(self, x_bf16, t_f32, n_valid, lr, mode=0, scale=1.0):
         m = x_bf16.shape[0]
+        if self._one_call(x_bf16, t_f32, m):
+            if m > self.batch:
+                self._alloc(m)
+            s = self._step()
+            tab = s.tensors
+            for i in range(2 * len(self.w)):
+                tab[i].weight_decay = 0.0
+            s.x, s.x_copy, s.target = x_bf16.data_ptr(), self.h[0].data_ptr(), t_f32.data_ptr()
+            s.m, s.nv, s.mode, s.scale, s.lr = m, n_valid, int(mode), float(scale), float(lr)
+            s.step = self.step_count + 1
+            _lib.check(self.lib.mcgb_mlp_train_step(C.byref(s), self._stream()))
+            self.step_count += 1
+            return self.loss_part[:(m + 255) // 256]
         y = self.forward(x_bf16, store=True)
         self.loss_grad(y, t_f32, m, n_valid, mode=mode, scale=scale)
         self.backward(self.grad_h[-1], m)
