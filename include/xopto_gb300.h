@@ -737,6 +737,30 @@ typedef struct McgbMlpStep {
 int mcgb_mlp_train_step(const McgbMlpStep *step, void *stream);
 uint64_t mcgb_mlp_train_scratch(const McgbAdamwTensor *tensors, int layers, int m);
 
+/* Profiles of m queries by a trained network (surrogate serving): inputs
+   scaled to [-1, 1] and split into high and low bf16 parts, the layers, and
+   profile b = exp(mu[b] + scale z[b]) in double precision.  queries holds
+   four rows of m doubles: mua, reduced scattering, g, n; the first two enter
+   by their logarithm.  Device pointers but for the struct itself; x [rows,
+   16], h[0] and h[1] [rows, widest hidden layer or 32] and z [rows, 32] are
+   scratch for rows = m rounded up to a multiple of 8.  widths[0] = 16,
+   widths[layers] = 32. */
+typedef struct McgbMlpPredict {
+    const uint16_t *w[MCGB_ADAMW_MAX_TENSORS / 2];
+    const float *b[MCGB_ADAMW_MAX_TENSORS / 2];
+    const double *queries;
+    const double *mu;                               /* [bins]                 */
+    uint16_t *x;
+    uint16_t *h[2];
+    float *z;
+    double *profiles;                               /* [m, bins]              */
+    double low[4], high[4], scale;
+    int32_t widths[MCGB_ADAMW_MAX_TENSORS / 2 + 1];
+    int32_t layers, m, bins;
+} McgbMlpPredict;
+
+int mcgb_mlp_predict(const McgbMlpPredict *p, void *stream);
+
 /* GEMM implementation behind the mcgb_mlp_* calls: 0 = tcgen05.mma on
    128 x 64 tiles with the FP32 accumulator in tensor memory (the default),
    1 = the warp-level mma.sync kernel on 64 x 64 tiles.  path = -1 only

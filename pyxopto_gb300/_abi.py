@@ -171,10 +171,18 @@ class McgbMlpStep(C.Structure):
                 ('scale', f32), ('lr', f32), ('beta1', f32), ('beta2', f32), ('eps', f32), ('reserved2', f32)]
 
 
+class McgbMlpPredict(C.Structure):
+    _fields_ = [('w', C.c_void_p * (ADAMW_MAX_TENSORS // 2)), ('b', C.c_void_p * (ADAMW_MAX_TENSORS // 2)),
+                ('queries', C.c_void_p), ('mu', C.c_void_p), ('x', C.c_void_p), ('h', C.c_void_p * 2),
+                ('z', C.c_void_p), ('profiles', C.c_void_p),
+                ('low', C.c_double * 4), ('high', C.c_double * 4), ('scale', C.c_double),
+                ('widths', i32 * (ADAMW_MAX_TENSORS // 2 + 1)), ('layers', i32), ('m', i32), ('bins', i32)]
+
+
 SIZEOF_KINDS = [McgbLayer, McgbSource, McgbDetector, McgbFluence, McgbTrace,
                 McgbMaterial, McgbMcmlConfig, McgbMcvoxConfig, McgbBuffers,
                 McgbRunOptions, McgbPf, McgbBatchSim, McgbBatchConfig, McgbSurface,
-                McgbSamplingVolume, McgbAdamwTensor, McgbMlpStep]
+                McgbSamplingVolume, McgbAdamwTensor, McgbMlpStep, McgbMlpPredict]
 
 
 def check_layout(sizeof_fn):

@@ -50,6 +50,7 @@ _OPTIONAL = {
     'mcgb_mlp_adamw_multi': (C.c_int, [_vp, C.c_int, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int,
                                        _vp]),
     'mcgb_mlp_train_step': (C.c_int, [C.POINTER(_abi.McgbMlpStep), _vp]),
+    'mcgb_mlp_predict': (C.c_int, [C.POINTER(_abi.McgbMlpPredict), _vp]),
     'mcgb_mlp_train_scratch': (C.c_uint64, [_vp, C.c_int, C.c_int]),
     'mcgb_mlp_loss_grad': (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int,
                                      C.c_float, _vp]),

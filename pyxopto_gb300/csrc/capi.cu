@@ -321,6 +321,7 @@ int mcgb_sizeof(int kind) {
         case 14: return (int)sizeof(McgbSamplingVolume);
         case 15: return (int)sizeof(McgbAdamwTensor);
         case 16: return (int)sizeof(McgbMlpStep);
+        case 17: return (int)sizeof(McgbMlpPredict);
         default: return -1;
     }
 }

@@ -375,21 +375,44 @@ class Surrogate:
         self.report['loss'] = hist
         return hist
 
+    # queries of one pass of predict(): bounds its device buffers (0.2 GB)
+    PREDICT_ROWS = 1 << 17
+
     def predict(self, mua, musr, g, n):
-        """Reflectance profiles [M, bins] for the given optical properties."""
+        """Reflectance profiles [M, bins] for the given optical properties.
+        The inputs and the exponential are computed on the device in double
+        precision."""
         import torch
-        x = features(mua, musr, g, n)
-        m = len(x)
-        mp = (m + 7) // 8 * 8
-        xp = np.zeros((mp, IN_PAD), np.float32)
-        xp[:m] = x
-        xd = split_bf16(xp)
-        out = []
-        for s in range(0, mp, self.mlp.batch):
-            z = self.mlp.forward(xd[s:s + self.mlp.batch], store=False)
-            out.append(z[:, :self.raxis.n].cpu().numpy().astype(np.float64))
-        z = np.concatenate(out)[:m]
-        return np.exp(self.mu[None, :] + self.scale * z)
+        m = len(np.asarray(mua))
+        q = np.empty((4, m))
+        for i, c in enumerate((mua, musr, g, n)):
+            q[i] = c
+        nb, net = self.raxis.n, self.mlp
+        if m == 0 or nb > OUT_PAD or not 1 <= len(net.w) <= _abi.ADAMW_MAX_TENSORS // 2:
+            raise ValueError('predict needs at least one query and at most {} bins'.format(OUT_PAD))
+        p = _abi.McgbMlpPredict()
+        nl = p.layers = len(net.w)
+        for i in range(nl):
+            p.w[i], p.b[i], p.widths[i] = net.wb[i].data_ptr(), net.b[i].data_ptr(), net.pads[i]
+        p.widths[nl] = net.pads[nl]
+        for i, k in enumerate(('log_mua', 'log_musr', 'g', 'n')):
+            p.low[i], p.high[i] = RANGES[k]
+        p.scale, p.bins = self.scale, nb
+        mu = torch.from_numpy(np.ascontiguousarray(self.mu, dtype=np.float64)).cuda()
+        most = min(m, self.PREDICT_ROWS)
+        rows = (most + 7) // 8 * 8
+        width = max(net.pads[1:])
+        x = torch.empty((rows, IN_PAD), dtype=torch.bfloat16, device='cuda')
+        h = torch.empty((2, rows, width), dtype=torch.bfloat16, device='cuda')
+        z = torch.empty((rows, OUT_PAD), dtype=torch.float32, device='cuda')
+        out = torch.empty((m, nb), dtype=torch.float64, device='cuda')
+        p.mu, p.x, p.z = mu.data_ptr(), x.data_ptr(), z.data_ptr()
+        p.h[0], p.h[1] = h[0].data_ptr(), h[1].data_ptr()
+        for s in range(0, m, most):
+            part = torch.from_numpy(np.ascontiguousarray(q[:, s:s + most])).cuda()
+            p.queries, p.m, p.profiles = part.data_ptr(), part.shape[1], out[s:].data_ptr()
+            _lib.check(net.lib.mcgb_mlp_predict(C.byref(p), net._stream()))
+        return out.cpu().numpy()
 
     # ------------------------------------------------------ weights
     def save(self, path):
