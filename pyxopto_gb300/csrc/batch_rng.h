@@ -32,7 +32,9 @@ BR_FN void br_packet_stream(uint64_t seed, uint32_t sim, uint64_t k, const uint3
                             uint32_t num_mult, uint64_t *x, uint32_t *a) {
     uint64_t h = br_splitmix64(seed ^ br_splitmix64(((uint64_t)sim << 40) ^ k));
     uint64_t h2 = br_splitmix64(h);
-    uint32_t m = mult[(uint32_t)(h2 % num_mult)];
+    /* the usual tables have a power of two of entries: no 64-bit division */
+    uint32_t pick = (num_mult & (num_mult - 1u)) ? (uint32_t)(h2 % num_mult) : (uint32_t)h2 & (num_mult - 1u);
+    uint32_t m = mult[pick];
     uint32_t c = (uint32_t)(h >> 32) % (m - 1u);
     uint32_t x0 = (uint32_t)h;
     if (x0 == 0xFFFFFFFFu) x0 = 0xFFFFFFFEu;

@@ -460,6 +460,7 @@ struct MlCtx {
 struct MlPacket {
     f3 pos, dir;
     float w, opl;
+    float pend;          /* deferred hits: the path that reaches a boundary, < 0 = none */
     int layer;
     uint32_t trace_count, events, steps;
     uint64_t p;          /* packet number (trace slot) */
@@ -487,6 +488,7 @@ static __device__ __forceinline__ void mcml_begin(const McgbMcmlConfig &c, const
                                                   const MlCtx &x, MlPacket &s, Rng &rng, uint64_t p) {
     s.p = p;
     s.opl = 0.0f;
+    s.pend = -1.0f;
     s.trace_count = 0;
     s.steps = 0;
     s.events = MCGB_EV_LAUNCH;
@@ -527,6 +529,60 @@ static __device__ __forceinline__ bool mcml_step_end(const McgbMcmlConfig &c, co
     return done;
 }
 
+/* Move to the boundary that the path reaches, reflect or refract there and
+   leave the sample or not (mcml.template.c:538-583, 668-704).  False when the
+   path ends inside the layer after all: then only the move is done. */
+template <bool XTRA>
+static __device__ __forceinline__ bool mcml_hit(const McgbMcmlConfig &c, const McgbBuffers &b,
+                                                const MlCtx &x, MlPacket &s, Rng &rng, float step,
+                                                bool &done) {
+    const MlLayer *L = x.L;
+    const float4 g0 = L[s.layer].g0;
+    int next = s.layer;
+    if (s.pos.z + step * s.dir.z < g0.x) {
+        --next;
+        if (fabsf(s.dir.z) != 0.0f) step = mc_div(g0.x - s.pos.z, s.dir.z);
+    }
+    if (s.pos.z + step * s.dir.z >= g0.y) {
+        ++next;
+        if (fabsf(s.dir.z) != 0.0f) step = mc_div(g0.y - s.pos.z, s.dir.z);
+    }
+    s.pos.x = s.pos.x + s.dir.x * step;
+    s.pos.y = s.pos.y + s.dir.y * step;
+    s.pos.z = s.pos.z + s.dir.z * step;
+    if (XTRA && x.track_opl) s.opl += L[s.layer].g1.x * step;
+    if (s.layer < next) s.pos.z = g0.y;
+    if (s.layer > next) s.pos.z = g0.x;
+    if (next == s.layer) return false;
+    uint32_t ev = mcml_boundary<XTRA>(c, x.lut, L, s.layer, next, x.last_layer, s.pos, s.dir, s.w, rng);
+    if (XTRA) s.events |= ev | MCGB_EV_BOUNDARY_HIT;
+    if (!(s.layer > 0 && s.layer < x.last_layer)) {
+        if (s.layer <= 0) detector_deposit<XTRA>(c.top, s.pos, s.dir, s.w, s.opl, b.accumulator, x.lut);
+        else detector_deposit<XTRA>(c.bottom, s.pos, s.dir, s.w, s.opl, b.accumulator, x.lut);
+        done = true;
+    }
+    return true;
+}
+
+/* Absorption, the new direction and the lottery (mcml.template.c:722-753). */
+template <bool FLU, bool XTRA>
+static __device__ __forceinline__ bool mcml_interact(const McgbMcmlConfig &c, MlPacket &s, Rng &rng,
+                                                     const Rng &srng, const f3 &sdir, float absorb, float mua,
+                                                     FluenceCache &fcache) {
+    float deposit = s.w * absorb;
+    s.w -= deposit;
+    if (XTRA) s.events |= MCGB_EV_ABSORPTION | MCGB_EV_SCATTERING;
+    if (FLU) fluence_deposit<XTRA>(c.fluence, s.pos, deposit, mua, fcache);
+    rng = srng;
+    s.dir = sdir;
+    if (s.w < c.opt.packet_weight_min) {
+        if (!c.opt.use_lottery) return true;
+        if (rng.next() > c.opt.lottery_chance) return true;
+        s.w = mc_div(s.w, c.opt.lottery_chance);
+    }
+    return false;
+}
+
 /* An albedo-weight step up to its end (mcml.template.c:525-753).  The
    direction after scattering is computed before it is known whether the
    path ends inside the layer: the random numbers that it takes are used up
@@ -535,14 +591,11 @@ static __device__ __forceinline__ bool mcml_step_end(const McgbMcmlConfig &c, co
    vain, and a warp pays for it anyway while one of its lanes scatters.  FAST
    math: 1e7 packets of the skin stack 53.7 -> 49.1 ms, 1e6 of the slab
    1.90 -> 1.70 ms. */
-template <int PF, bool FLU, bool XTRA>
+template <int PF, bool FLU, bool XTRA, bool DEFER = false>
 static __device__ __forceinline__ bool mcml_step_weight(const McgbMcmlConfig &c, const McgbBuffers &b,
                                                         const MlCtx &x, MlPacket &s, Rng &rng,
                                                         FluenceCache &fcache) {
-    const MlLayer *L = x.L;
-    const McgbRunOptions &o = c.opt;
-    uint64_t *accu = b.accumulator;
-    const MlLayer &cl = L[s.layer];
+    const MlLayer &cl = x.L[s.layer];
     const float4 g0 = cl.g0;   /* top, bottom, step factor, mua_inv_mut */
     ++s.steps;
     float u = rng.next();
@@ -553,54 +606,42 @@ static __device__ __forceinline__ bool mcml_step_weight(const McgbMcmlConfig &c,
     float step = sample_step(u, g0.z);
     step = fminf(step, FLT_MAX);
     float z = s.pos.z + step * s.dir.z;
-    if (z < g0.x || z >= g0.y) {
-        /* the path leaves the layer */
-        int next = s.layer;
-        if (z < g0.x) {
-            --next;
-            if (fabsf(s.dir.z) != 0.0f) step = mc_div(g0.x - s.pos.z, s.dir.z);
-        }
-        if (s.pos.z + step * s.dir.z >= g0.y) {
-            ++next;
-            if (fabsf(s.dir.z) != 0.0f) step = mc_div(g0.y - s.pos.z, s.dir.z);
-        }
-        s.pos.x = s.pos.x + s.dir.x * step;
-        s.pos.y = s.pos.y + s.dir.y * step;
-        s.pos.z = s.pos.z + s.dir.z * step;
-        if (XTRA && x.track_opl) s.opl += cl.g1.x * step;
-        if (s.layer < next) s.pos.z = g0.y;
-        if (s.layer > next) s.pos.z = g0.x;
-        if (next != s.layer) {
-            uint32_t ev = mcml_boundary<XTRA>(c, x.lut, L, s.layer, next, x.last_layer, s.pos, s.dir, s.w, rng);
-            if (XTRA) s.events |= ev | MCGB_EV_BOUNDARY_HIT;
-            if (!(s.layer > 0 && s.layer < x.last_layer)) {
-                if (s.layer <= 0) detector_deposit<XTRA>(c.top, s.pos, s.dir, s.w, s.opl, accu, x.lut);
-                else detector_deposit<XTRA>(c.bottom, s.pos, s.dir, s.w, s.opl, accu, x.lut);
-                return true;
-            }
+    if (DEFER) {
+        if (z < g0.x || z >= g0.y) {
+            s.pend = step;
             return false;
         }
-    } else {
-        s.pos.x = s.pos.x + s.dir.x * step;
-        s.pos.y = s.pos.y + s.dir.y * step;
-        s.pos.z = s.pos.z + s.dir.z * step;
-        if (XTRA && x.track_opl) s.opl += cl.g1.x * step;
+    } else if (z < g0.x || z >= g0.y) {
+        bool done = false;
+        if (mcml_hit<XTRA>(c, b, x, s, rng, step, done)) return done;
+        return mcml_interact<FLU, XTRA>(c, s, rng, srng, sdir, g0.w, cl.g1.y, fcache);
     }
-    float deposit = s.w * g0.w;
-    s.w -= deposit;
-    if (XTRA) s.events |= MCGB_EV_ABSORPTION | MCGB_EV_SCATTERING;
-    if (FLU) fluence_deposit<XTRA>(c.fluence, s.pos, deposit, cl.g1.y, fcache);
-    rng = srng;
-    s.dir = sdir;
-    if (s.w < o.packet_weight_min) {
-        if (o.use_lottery) {
-            if (rng.next() > o.lottery_chance) return true;
-            s.w = mc_div(s.w, o.lottery_chance);
-        } else {
-            return true;
-        }
-    }
-    return false;
+    s.pos.x = s.pos.x + s.dir.x * step;
+    s.pos.y = s.pos.y + s.dir.y * step;
+    s.pos.z = s.pos.z + s.dir.z * step;
+    if (XTRA && x.track_opl) s.opl += cl.g1.x * step;
+    return mcml_interact<FLU, XTRA>(c, s, rng, srng, sdir, g0.w, cl.g1.y, fcache);
+}
+
+/* The rest of a step whose path (s.pend) reaches a boundary.  Kept apart, so
+   that a warp runs it for the hits of several steps at once: on the skin
+   stack 1 % of a lane's steps hit a boundary but 29 % of a warp's, and each
+   cost the warp a hundred instructions for one or two lanes. */
+template <int PF, bool FLU, bool XTRA>
+static __device__ __forceinline__ bool mcml_deferred_hit(const McgbMcmlConfig &c, const McgbBuffers &b,
+                                                         const MlCtx &x, MlPacket &s, Rng &rng,
+                                                         FluenceCache &fcache) {
+    const float step = s.pend;
+    s.pend = -1.0f;
+    bool done = false;
+    if (mcml_hit<XTRA>(c, b, x, s, rng, step, done)) return done;
+    /* a layer of no thickness: the path ends inside after all */
+    const MlLayer &cl = x.L[s.layer];
+    Rng srng = rng;
+    f3 sdir = s.dir;
+    float az, ct = pf_sample<PF>(cl.pf0, cl.pf1, x.lut, srng, &az, sdir);
+    scatter_direction(sdir, ct, az);
+    return mcml_interact<FLU, XTRA>(c, s, rng, srng, sdir, cl.g0.w, cl.g1.y, fcache);
 }
 
 /* One interaction step of a packet (the body of McKernel's while(!done)
@@ -791,13 +832,13 @@ template <bool XTRA, class IO>
 static __device__ __forceinline__ void mcml_state(IO &io, MlPacket &s, Rng &rng) {
     io(s.pos.x); io(s.pos.y); io(s.pos.z);
     io(s.dir.x); io(s.dir.y); io(s.dir.z);
-    io(s.w); io(s.layer); io(s.steps);
+    io(s.w); io(s.pend); io(s.layer); io(s.steps);
     io(rng.x); io(rng.a);
     if (XTRA) {
         io(s.opl); io(s.trace_count); io(s.events); io(s.p);
     }
 }
-typedef WsExchange<17, ML_BLOCK / 32, 1, 8> MlExchange;
+typedef WsExchange<18, ML_BLOCK / 32, 1, 8> MlExchange;
 
 /* DYNAMIC scheduling: persistent warps refill idle lanes packet by packet
    from the queue counters[MCGB_CNT_QUEUE]; packet p runs on the stream of
@@ -852,11 +893,32 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
             need &= ~taken;
         }
         if (!more && !ws_share(share, active, [&](auto &io) { mcml_state<XTRA>(io, s, rng); })) break;
-        /* sixteen steps between refills; two steps per loop iteration give
-           the scheduler both bodies (+0.9 % on the layered stack) */
+        /* sixteen steps between refills, then their hits; two steps per loop
+           iteration give the scheduler both bodies.  Against hits in place,
+           after every 8 and 24 steps: 2e7 packets of the skin stack (FAST)
+           83.0 ms (88.9, 82.9, 85.9), 1e7 of the fibre 4.04 ms (4.87, 4.33,
+           3.93), 2e6 of the skin stack (EXACT) 23.8 ms (25.5, 23.2, 24.5). */
+        constexpr bool DEFER = METHOD == MCGB_METHOD_ALBEDO_WEIGHT && !XTRA;
 #pragma unroll 2
         for (int k = 0; k < 16; ++k) {
-            if (active && mcml_step<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status)) {
+            if (!active || (DEFER && s.pend >= 0.0f)) continue;
+            bool done;
+            if (DEFER) {
+                done = mcml_step_weight<PF, FLU, XTRA, true>(c, b, x, s, rng, fcache);
+                done = mcml_step_end<XTRA, XTRA || !SIMPLE>(c, b, x, s, status, done);
+            } else {
+                done = mcml_step<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status);
+            }
+            if (done) {
+                ++packets;
+                steps += s.steps;
+                mcml_end<XTRA>(c, b, x, s);
+                active = false;
+            }
+        }
+        if (DEFER && active && s.pend >= 0.0f) {
+            bool done = mcml_deferred_hit<PF, FLU, XTRA>(c, b, x, s, rng, fcache);
+            if (mcml_step_end<XTRA, XTRA || !SIMPLE>(c, b, x, s, status, done)) {
                 ++packets;
                 steps += s.steps;
                 mcml_end<XTRA>(c, b, x, s);
