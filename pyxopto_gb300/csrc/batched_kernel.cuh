@@ -318,10 +318,13 @@ batched_kernel(const McgbBatchConfig cfg, const uint32_t *__restrict__ mult,
         /* sixteen steps between refills, two step bodies per loop
            iteration: the refill's ballots and queue reads cost more than the
            idle lanes of a packet that ends early (+2.4 % against eight steps
-           without unrolling) */
+           without unrolling).  Once the queue is empty 64: the longest
+           packets are then a serial chain, which each try at the exchange
+           interrupts (32 simulations 101 -> 91 ms) */
         uint32_t taken = 0;
+        const uint32_t count = more ? 16u : 64u;
 #pragma unroll 2
-        for (int k = 0; k < 16; ++k) {
+        for (uint32_t k = 0; k < count; ++k) {
             if (active) {
                 ++taken;
                 if (batch_step<RMAX>(cfg, prep, c, s, rng, rmax2, tally)) {
@@ -331,8 +334,9 @@ batched_kernel(const McgbBatchConfig cfg, const uint32_t *__restrict__ mult,
             }
         }
         steps += taken;
-        iter += 16;
-        if ((iter & 1023u) == 0) {
+        iter += count;
+        if (iter >= 1024u) {
+            iter = 0;
             uint32_t stop = 0;
             if (lane == 0) {
                 if (globaltimer_ns() > t_deadline) stop = MCGB_STATUS_TIMEOUT;
