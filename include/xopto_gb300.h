@@ -536,6 +536,10 @@ int mcgb_fp32_fma_rate(uint32_t blocks, uint32_t threads, uint32_t iters, float 
 /* Fill a device uint64 buffer with a value (ScalarFillMcAccu). */
 int mcgb_fill_u64(uint64_t *dev, uint64_t n, uint64_t value, void *stream);
 
+/* dev_out[i] = dev_in[i] * scale in double precision: the integer tallies as
+   the host classes hold them (accumulator / K). */
+int mcgb_scale_u64(const uint64_t *dev_in, uint64_t n, double scale, double *dev_out, void *stream);
+
 /* Sampling volume of packet traces (replaces Mc.sampling_volume and its
    SamplingVolume kernel, xopto/mcml/mc.py:1040-1217,
    xopto/mcbase/kernel/mcsv.template.c:236-421).  For every packet the path

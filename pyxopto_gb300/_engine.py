@@ -46,7 +46,7 @@ class _Pool:
 
 def torch_cuda():
     import torch
-    if not torch.cuda.is_available():
+    if not torch.cuda.is_initialized() and not torch.cuda.is_available():
         raise RuntimeError('A CUDA device is required to run the GB300 simulator '
                            '(there is no CPU fallback).')
     return torch
@@ -242,11 +242,20 @@ class McEngine:
     # ----------------------------------------------------------- run cycle
     def _device_buffers(self, torch, device, lut: np.ndarray, extra: dict) -> _abi.McgbBuffers:
         d = self._dev
-        d['accu'] = torch.zeros((max(self._acc.size, 1),), dtype=torch.int64, device=device)
-        d['flt'] = torch.zeros((max(self._flt.size, 4),), dtype=torch.float32, device=device)
-        d['int'] = torch.zeros((max(self._int.size, 1),), dtype=torch.int32, device=device)
-        d['lut'] = torch.from_numpy(lut if lut.size else np.zeros((1,), np.float32)).to(device)
-        d['counters'] = torch.zeros((_abi.NUM_COUNTERS,), dtype=torch.int64, device=device)
+        # counters, tallies, trace events and counts in one zeroed block;
+        # each part starts on a 16-byte boundary
+        sizes = [_abi.NUM_COUNTERS * 8, max(self._acc.size, 1) * 8, max(self._flt.size, 4) * 4,
+                 max(self._int.size, 1) * 4]
+        starts = [0]
+        for n in sizes:
+            starts.append(starts[-1] + (n + 15) // 16 * 16)
+        block = torch.zeros((starts[-1] // 8,), dtype=torch.int64, device=device)
+        for key, dtype, at, n in zip(('counters', 'accu', 'flt', 'int'),
+                                     (torch.int64, torch.int64, torch.float32, torch.int32), starts, sizes):
+            part = block[at // 8:(at + (n + 7) // 8 * 8) // 8]
+            d[key] = part if dtype == torch.int64 else part.view(dtype)[:n // 4]
+        if lut.size:
+            d['lut'] = torch.from_numpy(lut).to(device)
         b = _abi.McgbBuffers()
         if 'dyn_mult' in d and extra.pop('_dynamic', False):
             b.rng_x = d['dyn_x'].data_ptr()
@@ -267,6 +276,53 @@ class McEngine:
         b.counters = d['counters'].data_ptr()
         return b
 
+    def _scaled(self, torch, tallies, scale: float) -> np.ndarray:
+        """Device tallies times ``scale`` as a host float64 array (converted
+        and multiplied on the device, mcgb_scale_u64)."""
+        out = torch.empty((tallies.numel(),), dtype=torch.float64, device=tallies.device)
+        _lib.check(_lib.load().mcgb_scale_u64(C.c_void_p(tallies.data_ptr()), tallies.numel(), float(scale),
+                                              C.c_void_p(out.data_ptr()),
+                                              C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        return out.cpu().numpy()
+
+    def _download(self, nphotons, out):
+        """The results of the latest launch: new (trace, fluence, detectors)
+        objects, or the ones in ``out`` updated."""
+        import torch
+        from .mcbase.mcdetector import Detectors, DetectorDefault
+        from .mcbase.mcfluence import Fluence
+        from .mcbase.mctrace import Trace
+        trace_res, fluence_res, detectors_res = out
+        if self._trace is not None:
+            flt = self._dev['flt'].cpu().numpy()
+            ints = self._dev['int'].cpu().numpy()
+            off, n = self._flt.find(self._trace)
+            ioff, ni = self._int.find(self._trace)
+            if trace_res is None:
+                trace_res = Trace(self._trace)
+            trace_res.update_data(self, flt[off:off + n], ints[ioff:ioff + ni], nphotons)
+        accu = self._dev['accu']
+        if self._fluence is not None:
+            off, n = self._acc.find(self._fluence)
+            if fluence_res is None:
+                fluence_res = Fluence(self._fluence)
+            if type(fluence_res).update_data is Fluence.update_data:
+                fluence_res.update_scaled(self._scaled(torch, accu[off:off + n], 1.0 / fluence_res.k), nphotons)
+            else:
+                fluence_res.update_data(self, [accu[off:off + n].cpu().numpy().view(np.uint64)], nphotons)
+        if self._detectors is not None:
+            if detectors_res is None:
+                detectors_res = Detectors(self._detectors)
+            used = [(det, res) for (_, det), (_, res) in zip(self._detectors.slots(), detectors_res.slots())
+                    if not isinstance(det, DetectorDefault)]
+            spans = [self._acc.find(det) for det, _ in used]
+            if spans:
+                first, last = min(off for off, _ in spans), max(off + n for off, n in spans)
+                host = accu[first:last].cpu().numpy().view(np.uint64)
+                for (_, res), (off, n) in zip(used, spans):
+                    res.update_data(self, [host[off - first:off - first + n]], nphotons)
+        return trace_res, fluence_res, detectors_res
+
     def sampling_volume(self, trace, sv, wgsize: int = None, maxthreads: int = None,
                         exportsrc=None, verbose: bool = False):
         """Adds the sampling volume of a trace to ``sv`` and returns it
@@ -277,6 +333,7 @@ class McEngine:
             raise RuntimeError('This Monte Carlo simulator was built without the Trace '
                                'functionality (the trace argument of Mc.__init__ was None)! '
                                'Sampling volume analysis requires trace functionality!')
+        from .mcbase.mcsv import SamplingVolume
         torch = torch_cuda()
         lib = _lib.load()
         t0 = time.perf_counter()
@@ -307,9 +364,12 @@ class McEngine:
                                        counters)
         t2 = time.perf_counter()
         _lib.check(code)
-        accu = d['sv_accu'].cpu().numpy().view(np.uint64)
         total = d['sv_total'].cpu().numpy().view(np.uint64)
-        sv.update_data(self, accumulators=[accu], nphotons=nphotons, total_weight=total)
+        if type(sv).update_data is SamplingVolume.update_data:
+            sv.update_scaled(self._scaled(torch, d['sv_accu'], sv.scale(self)), total)
+        else:
+            sv.update_data(self, accumulators=[d['sv_accu'].cpu().numpy().view(np.uint64)],
+                           nphotons=nphotons, total_weight=total)
         t3 = time.perf_counter()
         self._run_report.update(upload=t1 - t0, execution=t2 - t1, download=t3 - t2,
                                 items=nphotons, threads=None)

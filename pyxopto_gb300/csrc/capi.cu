@@ -281,6 +281,14 @@ __global__ void __launch_bounds__(1024) fma_rate_kernel(uint32_t iters, float *o
     if (s == -1.0f) out[blockIdx.x] = s;
 }
 
+/* out[i] = in[i] * scale in double precision, the conversion and the product
+   each rounded, as numpy evaluates it. */
+__global__ void scale_u64_kernel(const uint64_t *__restrict__ in, uint64_t n, double scale, double *__restrict__ out) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x)
+        out[i] = __dmul_rn(__ull2double_rn(in[i]), scale);
+}
+
 __global__ void fill_u64_kernel(uint64_t *p, uint64_t n, uint64_t v) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x)
@@ -464,6 +472,16 @@ int mcgb_fp32_fma_rate(uint32_t blocks, uint32_t threads, uint32_t iters, float 
     fma_rate_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(iters, dev_out);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MCGB_OK : cuda_fail(e, "fma probe launch");
+}
+
+int mcgb_scale_u64(const uint64_t *dev_in, uint64_t n, double scale, double *dev_out, void *stream) {
+    if (n == 0) return MCGB_OK;
+    if (!dev_in || !dev_out) return fail(MCGB_E_INVALID, "NULL tally array");
+    uint64_t blocks = (n + 255) / 256;
+    if (blocks > 152u * 16u) blocks = 152u * 16u;
+    scale_u64_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(dev_in, n, scale, dev_out);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? MCGB_OK : cuda_fail(e, "tally scaling");
 }
 
 int mcgb_fill_u64(uint64_t *dev, uint64_t n, uint64_t value, void *stream) {

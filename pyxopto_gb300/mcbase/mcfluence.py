@@ -54,12 +54,16 @@ class Fluence:
     data = property(_get_data, None, None, 'Deposition or fluence rate per packet and volume.')
 
     def update_data(self, mc, accumulators, nphotons: int, **kwargs):
-        acc = np.asarray(accumulators[0]).reshape(self.shape)
+        self.update_scaled(np.asarray(accumulators[0]) * (1.0 / self._k), nphotons)
+
+    def update_scaled(self, scaled: np.ndarray, nphotons: int):
+        """update_data for tallies already multiplied by 1/k."""
+        scaled = scaled.reshape(self.shape)
         if self._data is not None:
-            self._data += acc * (1.0 / self._k)
+            self._data += scaled
             self._nphotons += int(nphotons)
         else:
-            self._data = acc * (1.0 / self._k)
+            self._data = scaled
             self._nphotons = int(nphotons)
 
     def update(self, obj: 'Fluence'):

@@ -85,9 +85,15 @@ class SamplingVolume:
 
     def update_data(self, mc, accumulators, total_weight, **kwargs):
         """Adds the raw tallies scaled by 1/(k * multiplier) (mcsv.py:313-342)."""
-        multiplier = self._multiplier(mc)
-        new = np.reshape(np.asarray(accumulators[0], dtype=np.float64), self.shape) * \
-            (1.0 / (self._k * multiplier))
+        self.update_scaled(np.asarray(accumulators[0], dtype=np.float64) * self.scale(mc), total_weight)
+
+    def scale(self, mc=None) -> float:
+        """The value of one unit of the raw tallies."""
+        return 1.0 / (self._k * self._multiplier(mc))
+
+    def update_scaled(self, scaled: np.ndarray, total_weight):
+        """update_data for tallies already multiplied by ``scale``."""
+        new = np.reshape(scaled, self.shape)
         w = float(np.asarray(total_weight).ravel()[0]) / self._k
         if self._data is not None:
             self._data += new

@@ -154,32 +154,6 @@ class Mc(McEngine):
         buffers = self._device_buffers(torch, device, self._lut_array(), {'_dynamic': dynamic})
         return lib.mcgb_mcml_run, cfg, buffers
 
-    def _download(self, nphotons, out):
-        accu = self._dev['accu'].cpu().numpy().view(np.uint64)
-        trace_res, fluence_res, detectors_res = out
-        if self._trace is not None:
-            flt = self._dev['flt'].cpu().numpy()
-            ints = self._dev['int'].cpu().numpy()
-            off, n = self._flt.find(self._trace)
-            ioff, ni = self._int.find(self._trace)
-            if trace_res is None:
-                trace_res = mctrace.Trace(self._trace)
-            trace_res.update_data(self, flt[off:off + n], ints[ioff:ioff + ni], nphotons)
-        if self._fluence is not None:
-            off, n = self._acc.find(self._fluence)
-            if fluence_res is None:
-                fluence_res = mcfluence.Fluence(self._fluence)
-            fluence_res.update_data(self, [accu[off:off + n]], nphotons)
-        if self._detectors is not None:
-            if detectors_res is None:
-                detectors_res = mcdetector.Detectors(self._detectors)
-            for (slot, det), (_, res) in zip(self._detectors.slots(), detectors_res.slots()):
-                if isinstance(det, mcdetector.DetectorDefault):
-                    continue
-                off, n = self._acc.find(det)
-                res.update_data(self, [accu[off:off + n]], nphotons)
-        return trace_res, fluence_res, detectors_res
-
     def rng_test(self, n: int, x: int = None, a: int = None) -> np.ndarray:
         """n uniform random numbers of one stream computed on the device
         (Mc.rng_test, xopto/mcml/mc.py:1320-1362)."""

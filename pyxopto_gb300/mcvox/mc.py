@@ -16,6 +16,9 @@ from ..mcbase.mcutil import Axis, RadialAxis
 from . import (mcgeometry, mcsource, mcdetector, mcpf, mcfluence, mctrace, mcoptions, mctypes,
                mcmaterial, mcsv, mcsurface)
 
+_memcmp = C.CDLL(None).memcmp
+_memcmp.argtypes, _memcmp.restype = [C.c_void_p, C.c_void_p, C.c_size_t], C.c_int
+
 
 class Mc(McEngine):
     MEDIUM = 1
@@ -54,6 +57,16 @@ class Mc(McEngine):
             material_index = int(self._voxels[ind])
         return self._materials[material_index]
 
+    def _kept_voxels(self):
+        """(a copy of the material indices, the largest of them), taken anew
+        when their shape or content has changed since the last call."""
+        vox = np.ascontiguousarray(self._voxels.data(), dtype=np.uint8)
+        kept = getattr(self, '_kept', None)
+        if kept is None or kept[0].shape != vox.shape or \
+                _memcmp(kept[0].ctypes.data, vox.ctypes.data, vox.nbytes) != 0:
+            kept = self._kept = (vox.copy(), int(vox.max()) if vox.size else -1)
+        return kept
+
     def pack(self, nphotons: int, num_streams: int = 1):
         """Returns (config, material table) in C-ABI form."""
         self._clear_allocators()
@@ -64,10 +77,9 @@ class Mc(McEngine):
         if type(self._source) != self._source_type:
             raise ValueError('The photon packet source type/kind must not change '
                              'between simulation calls!')
-        data = self._voxels.data()
-        if data.size and int(data.max()) >= len(self._materials):
+        if self._kept_voxels()[1] >= len(self._materials):
             raise ValueError('Voxel material index {} is outside the material list of length '
-                             '{}!'.format(int(data.max()), len(self._materials)))
+                             '{}!'.format(self._kept_voxels()[1], len(self._materials)))
         cfg = _abi.McgbMcvoxConfig()
         cfg.num_packets = int(nphotons)
         cfg.num_streams = int(num_streams)
@@ -138,11 +150,10 @@ class Mc(McEngine):
                 else max(1, int(maxthreads))
             self._ensure_streams(torch, n_streams, device)
             cfg.num_streams = n_streams
-        vox = np.ascontiguousarray(self._voxels.data(), dtype=np.uint8)
-        key = (vox.shape, hash(vox.tobytes()))
-        if self._dev.get('vox_key') != key:
-            self._dev['vox'] = torch.from_numpy(vox.reshape(-1).copy()).to(device)
-            self._dev['vox_key'] = key
+        vox = self._kept[0]
+        if self._dev.get('vox_of') is not vox:
+            self._dev['vox'] = torch.from_numpy(vox.reshape(-1)).to(device)
+            self._dev['vox_of'] = vox
             self._dev.pop('vox_radius', None)
         radius = None
         if cfg.opt.math == _abi.MATH_FAST and self._free_flight():
@@ -175,32 +186,6 @@ class Mc(McEngine):
             self._dev['vox_radius'] = rad if int(rad.max().item()) > 0 else None
         rad = self._dev['vox_radius']
         return rad.data_ptr() if rad is not None else None
-
-    def _download(self, nphotons, out):
-        accu = self._dev['accu'].cpu().numpy().view(np.uint64)
-        trace_res, fluence_res, detectors_res = out
-        if self._trace is not None:
-            flt = self._dev['flt'].cpu().numpy()
-            ints = self._dev['int'].cpu().numpy()
-            off, n = self._flt.find(self._trace)
-            ioff, ni = self._int.find(self._trace)
-            if trace_res is None:
-                trace_res = mctrace.Trace(self._trace)
-            trace_res.update_data(self, flt[off:off + n], ints[ioff:ioff + ni], nphotons)
-        if self._fluence is not None:
-            off, n = self._acc.find(self._fluence)
-            if fluence_res is None:
-                fluence_res = mcfluence.Fluence(self._fluence)
-            fluence_res.update_data(self, [accu[off:off + n]], nphotons)
-        if self._detectors is not None:
-            if detectors_res is None:
-                detectors_res = mcdetector.Detectors(self._detectors)
-            for (slot, det), (_, res) in zip(self._detectors.slots(), detectors_res.slots()):
-                if isinstance(det, mcdetector.DetectorDefault):
-                    continue
-                off, n = self._acc.find(det)
-                res.update_data(self, [accu[off:off + n]], nphotons)
-        return trace_res, fluence_res, detectors_res
 
     def __str__(self):
         return 'Mc(voxels={}, materials={}, source={})'.format(
