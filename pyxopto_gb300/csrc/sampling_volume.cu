@@ -13,12 +13,19 @@
 // integers updated with atomics; a 200^3 volume is 64 MB and stays in L2.
 //
 // Compiled without contraction (-fmad=false) and with IEEE division and
-// square root: the walk compares distances, and a fused multiply-add would
-// move a crossing to another voxel.
+// square root (exact_math.cuh): the walk compares distances, and a fused
+// multiply-add would move a crossing to another voxel.
+//
+// What bounds it is the longest walk: a serial chain of event loads, three
+// divisions per wall and a square root per event, on a few warps.  The event
+// after the next is loaded while the walk is on its way to the next one, the
+// divisions share one range test, and short traces put a few packets into
+// each warp of the whole chip instead of 32 into a few of them.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/xopto_gb300.h"
+#include "exact_math.cuh"
 
 namespace {
 
@@ -39,7 +46,7 @@ __device__ __forceinline__ void sv_load(const float *packet, int32_t i, SvEvent 
 // mc_distance_fpv3 (xopto/mcbase/kernel/mcbase.template.c:1061-1064).
 __device__ __forceinline__ float sv_distance(const SvEvent &a, const SvEvent &b) {
     float x = a.px - b.px, y = a.py - b.py, z = a.pz - b.pz;
-    return sqrtf(x * x + y * y + z * z);
+    return em_sqrt(x * x + y * y + z * z);
 }
 
 // Float to integer conversions truncate toward zero and saturate (a negative
@@ -52,20 +59,42 @@ struct SvVoxel {
 
 // sva_intersect (mcsv.template.c:97-120): distance along the direction to the
 // exit wall of the current voxel on each axis.
-__device__ __forceinline__ float sv_wall(float top_left, int32_t v, float size, float pos,
-                                         float dir) {
-    float d = top_left + (float)((int32_t)(dir >= 0.0f) + v) * size - pos;
-    return dir != 0.0f ? d / dir : __int_as_float(0x7f800000);
+__device__ __forceinline__ float sv_gap(float top_left, int32_t v, float size, float pos, float dir) {
+    return top_left + (float)((int32_t)(dir >= 0.0f) + v) * size - pos;
+}
+
+__device__ __forceinline__ void sv_walls(const McgbSamplingVolume &sv, const SvVoxel &v, const SvEvent &e,
+                                         float &dx, float &dy, float &dz) {
+    const float gx = sv_gap(sv.top_left[0], v.x, sv.voxel_size[0], e.px, e.dx);
+    const float gy = sv_gap(sv.top_left[1], v.y, sv.voxel_size[1], e.py, e.dy);
+    const float gz = sv_gap(sv.top_left[2], v.z, sv.voxel_size[2], e.pz, e.dz);
+    const float least = fminf(fminf(fabsf(gx), fminf(fabsf(gy), fabsf(gz))),
+                              fminf(fabsf(e.dx), fminf(fabsf(e.dy), fabsf(e.dz))));
+    const float most = fmaxf(fmaxf(fabsf(gx), fmaxf(fabsf(gy), fabsf(gz))),
+                             fmaxf(fabsf(e.dx), fmaxf(fabsf(e.dy), fabsf(e.dz))));
+    if (least >= EM_LO && most <= EM_HI) {
+        dx = em_quot(gx, e.dx, em_recip(e.dx));
+        dy = em_quot(gy, e.dy, em_recip(e.dy));
+        dz = em_quot(gz, e.dz, em_recip(e.dz));
+    } else {
+        const float inf = __int_as_float(0x7f800000);
+        dx = e.dx != 0.0f ? gx / e.dx : inf;
+        dy = e.dy != 0.0f ? gy / e.dy : inf;
+        dz = e.dz != 0.0f ? gz / e.dz : inf;
+    }
 }
 
 __global__ void __launch_bounds__(128)
 sampling_volume_kernel(McgbSamplingVolume sv, const float *__restrict__ trace,
                        const int32_t *__restrict__ counts, uint64_t *__restrict__ accu,
-                       uint64_t *__restrict__ total_weight, uint64_t *__restrict__ counters) {
+                       uint64_t *__restrict__ total_weight, uint64_t *__restrict__ counters,
+                       uint32_t per_warp) {
     const float k = (float)sv.k;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < sv.num_packets;
-         p += stride) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane >= per_warp) return;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32u;
+    const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x / 32u) * per_warp;
+    for (uint64_t p = warp * per_warp + lane; p < sv.num_packets; p += stride) {
         int32_t n = counts[p];
         if (n > (int32_t)sv.max_events) n = (int32_t)sv.max_events;
         if (n <= 0) continue;
@@ -75,10 +104,11 @@ sampling_volume_kernel(McgbSamplingVolume sv, const float *__restrict__ trace,
         atomicAdd((unsigned long long *)total_weight,
                   (unsigned long long)sv_weight(end_w * k + 0.5f));
 
-        SvEvent e1, e2;
+        SvEvent e1, e2, e3;   /* the event left behind, the next, the one after */
         int32_t ei = 0;
         sv_load(tr, 0, e1);
         sv_load(tr, n > 1 ? 1 : n - 1, e2);
+        sv_load(tr, n > 2 ? 2 : n - 1, e3);
         float d12 = sv_distance(e1, e2);
         SvVoxel v;
         v.x = __float2int_rz((e1.px - sv.top_left[0]) / sv.voxel_size[0]);
@@ -88,9 +118,8 @@ sampling_volume_kernel(McgbSamplingVolume sv, const float *__restrict__ trace,
         uint32_t crossings = 0;
 
         while (true) {
-            float dx = sv_wall(sv.top_left[0], v.x, sv.voxel_size[0], e1.px, e1.dx);
-            float dy = sv_wall(sv.top_left[1], v.y, sv.voxel_size[1], e1.py, e1.dy);
-            float dz = sv_wall(sv.top_left[2], v.z, sv.voxel_size[2], e1.pz, e1.dz);
+            float dx, dy, dz;
+            sv_walls(sv, v, e1, dx, dy, dz);
             float d_voxel = fminf(dz, fminf(dx, dy));
             float d_move = fminf(d_voxel, d12);
             l_voxel += d_move;
@@ -100,7 +129,8 @@ sampling_volume_kernel(McgbSamplingVolume sv, const float *__restrict__ trace,
                 e1 = e2;
                 ++ei;
                 if (ei < n - 1) {
-                    sv_load(tr, ei + 1, e2);
+                    e2 = e3;
+                    if (ei + 2 < n) sv_load(tr, ei + 2, e3);
                     d12 = sv_distance(e1, e2);
                     continue;
                 }
@@ -153,11 +183,17 @@ cudaError_t launch(const McgbSamplingVolume &sv, const float *trace, const int32
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
-    uint64_t blocks = (sv.num_packets + 127) / 128;
+    /* packets per warp: lanes diverge between events and walls, so an even
+       share over twelve warps of every SM, at most all lanes (5,000 traces of
+       500 events 2.06 -> 0.96 ms; over four warps 1.11, over 32 1.01) */
+    const uint64_t warps = 12u * (uint64_t)(sms > 0 ? sms : 1);
+    uint64_t per_warp = (sv.num_packets + warps - 1) / warps;
+    if (per_warp > 32) per_warp = 32;
+    uint64_t blocks = (sv.num_packets + 4 * per_warp - 1) / (4 * per_warp);
     uint64_t cap = (uint64_t)(sms > 0 ? sms : 1) * 16;
     if (blocks > cap) blocks = cap;
-    sampling_volume_kernel<<<(unsigned)blocks, 128, 0, stream>>>(sv, trace, counts, accu,
-                                                                total_weight, counters);
+    sampling_volume_kernel<<<(unsigned)blocks, 128, 0, stream>>>(sv, trace, counts, accu, total_weight, counters,
+                                                                (uint32_t)per_warp);
     return cudaGetLastError();
 }
 
