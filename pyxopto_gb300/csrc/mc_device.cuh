@@ -252,9 +252,9 @@ MCGB_DEV void scatter_direction(f3 &dir, float cos_theta, float fi) {
     y = along ? stsf : y;
     z = along ? zs : z;
     float r2 = x * x + y * y + z * z;
-    float r = em_recip(em_sqrt_normal(r2));
+    float r = em_rcp_length_near1(r2);
     const float least = along ? 1.0f : fminf(fabsf(nx), fabsf(ny));
-    if (fminf(fminf(st2, least), r2) >= EM_LO && r2 <= EM_HI)
+    if (fminf(st2, least) >= EM_LO && fabsf(r2 - 1.0f) <= 0.000244140625f)
         dir = f3{x * r, y * r, z * r};
     else
         dir = scatter_direction_ieee(dir, cos_theta, fi);

@@ -90,6 +90,10 @@ static __device__ uint32_t check(int op, u64 i) {
         return !same(em_log_uniform(u), pm_logf(u)) + !same(s, ps) + !same(c, pc);
     }
     if (op == 6) return !same(em_exp(__uint_as_float((uint32_t)i)), pm_expf(__uint_as_float((uint32_t)i)));
+    if (op == 8) {            /* every float within 2^-12 of 1 */
+        float x = __uint_as_float(0x3f7ff000u + (uint32_t)i);
+        return fabsf(x - 1.0f) <= 0.000244140625f && !same(em_rcp_length_near1(x), 1.0f / sqrtf(x));
+    }
     float x = __uint_as_float((uint32_t)(i >> 4) * 2654435761u);
     const float ys[16] = {-1.0f, -0.5f, -2.0f, 0.0f, 1.0f, 0.333333343f, -0.833333313f, -1.0e3f,
                           2.0f, -10.0f, 0.0769230798f, -4.0f, 1e-30f, -1e30f, -3.4e38f, 1.5f};
@@ -137,6 +141,7 @@ def probe(cuda, tmp_path_factory):
     pytest.param(0, 1 << 23, id='reciprocal'), pytest.param(1, 1 << 23, id='sqrt'),
     pytest.param(2, 1 << 23, id='quotients at midpoints'), pytest.param(3, 1 << 32, id='quotients'),
     pytest.param(4, 1 << 32, id='log'), pytest.param(5, 1 << 32, id='uniform log and azimuth'),
-    pytest.param(6, 1 << 32, id='exp'), pytest.param(7, 1 << 32, id='powr')])
+    pytest.param(6, 1 << 32, id='exp'), pytest.param(7, 1 << 32, id='powr'),
+    pytest.param(8, 1 << 13, id='length near 1')])
 def test_device_arithmetic_equals_ieee_and_portable(probe, op, count):
     assert probe(op, count) == 0
