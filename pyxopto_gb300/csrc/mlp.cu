@@ -626,12 +626,13 @@ int mcgb_mlp_predict(const McgbMlpPredict *p, void *stream) {
 
 uint64_t mcgb_mlp_train_scratch(const McgbAdamwTensor *tensors, int layers, int m) {
     if (!tensors || layers < 1 || layers > STEP_MAX_LAYERS || m <= 0) return 0;
-    const uint64_t groups = (uint64_t)(m + 31) / 32;
+    const uint64_t groups = (uint64_t)(m + 31) / 32, chunks = (uint64_t)(m + 63) / 64;
     uint64_t n = (2 * groups + 3) / 4 * 4;
     for (int i = 0; i < layers; ++i) {
-        int rows, parts, slices;
-        step_slices(tensors[2 * i], m, step_tiles(tensors, layers), rows, parts, slices);
-        n += (uint64_t)slices * tensors[2 * i].rows * tensors[2 * i].cols + groups * (uint64_t)tensors[2 * i].rows;
+        int rows, count;
+        step_slices(tensors[2 * i], m, rows, count);
+        n += (uint64_t)(count < 8 ? count : 8) * tensors[2 * i].rows * tensors[2 * i].cols +
+             chunks * (uint64_t)tensors[2 * i].rows;
     }
     return n;
 }
@@ -662,8 +663,8 @@ int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
     if (all & 15u) return fail(MCGB_E_INVALID, "train_step operands must be 16-byte aligned");
 
     cudaStream_t st = (cudaStream_t)stream;
-    int rows[STEP_MAX_LAYERS], parts[STEP_MAX_LAYERS], slices[STEP_MAX_LAYERS];
-    const int groups = (m + 31) / 32;
+    int rows[STEP_MAX_LAYERS], count[STEP_MAX_LAYERS], slices[STEP_MAX_LAYERS];
+    const int groups = (m + 31) / 32, chunks = (m + 63) / 64;
     float *at = s->scratch;
     float *loss_part = at;
     at += (2 * groups + 3) / 4 * 4;
@@ -671,13 +672,14 @@ int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
     memset(&up, 0, sizeof(up));
     float *dw[STEP_MAX_LAYERS], *db[STEP_MAX_LAYERS];
     for (int i = 0; i < L; ++i) {
-        step_slices(t[2 * i], m, step_tiles(t, L), rows[i], parts[i], slices[i]);
+        step_slices(t[2 * i], m, rows[i], count[i]);
+        slices[i] = count[i] < 8 ? count[i] : 8;
         dw[i] = at;
         at += (size_t)slices[i] * t[2 * i].rows * t[2 * i].cols;
     }
     for (int i = 0; i < L; ++i) {
         db[i] = at;
-        at += (size_t)groups * t[2 * i].rows;
+        at += (size_t)chunks * t[2 * i].rows;
     }
     const int mt = (m + TBM - 1) / TBM;
     auto wide = [&](int cols) { return (long)mt * ((cols + 63) / 64) >= sm_count(); };
@@ -741,11 +743,11 @@ int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
             l.k = t[2 * i].cols;
             l.first = first;
             l.rows = rows[i];
-            l.parts = parts[i];
-            l.slices = slices[i];
-            first += slices[i] * ((l.n + TBM - 1) / TBM) * ((l.k + STEP_BN - 1) / STEP_BN);
+            l.count = count[i];
+            const int width = step_width(l.count);
+            first += slices[i] * ((l.n + TBM - 1) / TBM) * ((l.k + width - 1) / width);
         }
-        e = step_launch_tc(step_weights, TcShape<STEP_BN>::SMEM, dim3(first), st, f);
+        e = step_launch_tc(step_weights, TcShape<64>::SMEM, dim3(first), st, f);
     }
     if (e == cudaSuccess) {
         up.a.count = 2 * L;
@@ -765,7 +767,7 @@ int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
         }
         up.weights = up.wstart[L];
         up.layers = L;
-        up.groups = groups;
+        up.chunks = chunks;
         up.tie_count = s->tie_count;
         up.tie_shift = s->tie_shift;
         up.loss_part = loss_part;

@@ -16,39 +16,48 @@
  *   step_backward  per hidden layer: dPre W, times GELU', and column sums
  *   step_weights   every layer: dPre^T X over slices of the rows
  *   step_update    slice sums, tied columns, AdamW, bf16 and transposed copies
- * The products, roundings and per-element formulas are those of the separate
- * kernels; only the order of the FP32 sums over rows differs.
+ * The products, roundings, formulas and sums are those of the separate
+ * kernels, bit for bit; only the loss is summed in another order.
  * A step, the Python call included: batch 256 205 -> 53 us, 4096 208 -> 87 us,
- * 16384 295 -> 209 us.  Weight gradients in the separate kernel's slices (32
- * to 64 a layer, 18 MB of partial sums at 4096) cost 30 us more; 64 x wide
- * tiles throughout 10 us more at 256.
+ * 16384 296 -> 236 us.  A block and partial sum for each of the separate
+ * kernel's slices (32 to 64 a layer, 18 MB of partial sums at 4096) cost 30 us
+ * more; other sums (slices as long as fill the SMs once) 27 us less at 16384
+ * and nothing at 4096, but biases that differ by an ulp flip bf16 roundings
+ * of the next step.
  */
 #pragma once
 
 constexpr int STEP_MAX_LAYERS = MCGB_ADAMW_MAX_TENSORS / 2;
 
-/* Sums over the 32 lanes of 16 columns per lane; lane l returns column l / 2
-   of the 16. */
-__device__ __forceinline__ float warp_columns16(float (&v)[16]) {
-    const int lane = threadIdx.x & 31;
+/* Column sums of a 128 x BN tile of dPre that the block has written to shared
+   memory ([row][column], rows of BN + 1), as act_bwd_kernel takes them: for
+   each 64 rows the sums over rows 8 apart, then those eight in order. */
+template <int BN>
+__device__ __forceinline__ void store_columns(float *tile, float *part, int r0, int c0, int ldc, int R) {
+    float *red = tile + TBM * (BN + 1);   /* [chunk][row mod 8][column] */
+    __syncthreads();
+    for (int e = threadIdx.x; e < 16 * BN; e += TNT) {
+        const int c = e % BN, row = e / BN / 8 * 64 + e / BN % 8;
+        float s = 0.0f;
 #pragma unroll
-    for (int d = 16, n = 8; n >= 1; d >>= 1, n >>= 1) {
-        const bool up = (lane & d) != 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (q >= n) continue;
-            const float keep = up ? v[q + n] : v[q], send = up ? v[q] : v[q + n];
-            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-        }
+        for (int q = 0; q < 8; ++q) s += tile[(row + 8 * q) * (BN + 1) + c];
+        red[e] = s;
     }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+    __syncthreads();
+    for (int e = threadIdx.x; e < 2 * BN; e += TNT) {
+        const int c = e % BN, row = r0 + e / BN * 64;
+        float t = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += red[(e / BN * 8 + q) * BN + c];
+        if (row < R && c0 + c < ldc) part[(size_t)(row / 64) * ldc + c0 + c] = t;
+    }
 }
 
-/* Stores the warp's column sums of dPre: part[row / 32][column]. */
-__device__ __forceinline__ void store_columns(float (&v)[16], float *part, int r0, int c, int ldc, int R) {
-    const float s = warp_columns16(v);
-    const int lane = threadIdx.x & 31, row = r0 + (int)(threadIdx.x & 96u);
-    if (row < R && (lane & 1) == 0) part[(size_t)(row / 32) * ldc + c + (lane >> 1)] = s;
+/* The shared memory of the operand stages, free once the product is done. */
+template <int BN>
+__device__ __forceinline__ float *step_tile(uint8_t *tc_smem) {
+    static_assert((TBM * (BN + 1) + 16 * BN) * 4 <= TcShape<BN>::BARS, "column sums fit the stages");
+    return reinterpret_cast<float *>(tc_smem);
 }
 
 struct StepForward {
@@ -79,6 +88,7 @@ __global__ void __launch_bounds__(TNT) step_forward(const __grid_constant__ Step
         for (int q = 0; q < p.k / 8; ++q) to[q] = from[q];
     }
     const float inv = 1.0f / ((float)p.m * (float)p.nv);
+    float *tile = step_tile<BN>(tc_smem);
     float loss = 0.0f;
 #pragma unroll 1
     for (int j = threadIdx.x >> 7; j < BN / 16; j += TNT / 128) {
@@ -117,7 +127,8 @@ __global__ void __launch_bounds__(TNT) step_forward(const __grid_constant__ Step
                 tc_store16(p.h + o, v);
                 tc_store16(p.dpre + o, t);
             }
-            store_columns(t, p.part, r0, c, p.n, p.m);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) tile[tc_row() * (BN + 1) + j * 16 + q] = t[q];
         } else if (in) {
             if (p.act) {
 #pragma unroll
@@ -131,6 +142,7 @@ __global__ void __launch_bounds__(TNT) step_forward(const __grid_constant__ Step
         for (int d = 16; d > 0; d >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, d);
         const int row = r0 + (int)(threadIdx.x & 96u);
         if ((threadIdx.x & 31) == 0 && row < p.m) p.loss_part[row / 32 * 2 + (threadIdx.x >> 7)] = loss;
+        store_columns<BN>(tile, p.part, r0, c0, p.n, p.m);
     }
     tc_release<BN>(tmem);
 }
@@ -150,6 +162,7 @@ __global__ void __launch_bounds__(TNT) step_backward(const __grid_constant__ Ste
     uint32_t tmem;
     const bool ok = tc_product<BN, false, false>(tc_smem, p.dpre, p.n, p.wt, p.n, p.m, p.k, r0, c0, 0, p.n, tmem);
     const int r = r0 + tc_row();
+    float *tile = step_tile<BN>(tc_smem);
 #pragma unroll 1
     for (int j = threadIdx.x >> 7; j < BN / 16; j += TNT / 128) {
         const int c = c0 + j * 16;
@@ -171,20 +184,20 @@ __global__ void __launch_bounds__(TNT) step_backward(const __grid_constant__ Ste
 #pragma unroll
             for (int q = 0; q < 16; ++q) v[q] = 0.0f;
         }
-        store_columns(v, p.part, r0, c, p.k, p.m);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) tile[tc_row() * (BN + 1) + j * 16 + q] = v[q];
     }
+    store_columns<BN>(tile, p.part, r0, c0, p.k, p.m);
     tc_release<BN>(tmem);
 }
 
-constexpr int STEP_BN = 64;     /* columns of a weight-gradient tile */
-constexpr int STEP_PARTS = 4;   /* accumulators of a weight-gradient CTA */
+constexpr int STEP_COLS = 256;   /* accumulator columns of a weight-gradient CTA */
 
 struct StepWeightLayer {
     const bf16 *dpre, *x;   /* [m, n], [m, k] */
-    float *out;             /* [slices][n][k] */
+    float *out;             /* [min(count, 8)][n][k] */
     int n, k, first;        /* first block */
-    int rows, slices;       /* rows per accumulator; slices of STEP_PARTS or fewer of them */
-    int parts;
+    int rows, count;        /* the slices of mcgb_mlp_linear_bwd_weight */
 };
 
 struct StepWeights {
@@ -192,65 +205,71 @@ struct StepWeights {
     int layers, m;
 };
 
-/* A CTA sums over more rows than the separate kernel's slices, so that the
-   partial sums stay few, but in an accumulator of its own for each of those
-   slices: no FP32 sum in the tensor core gets longer. */
-__global__ void __launch_bounds__(TNT) step_weights(const __grid_constant__ StepWeights p) {
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
-    int i = p.layers - 1;
-    while (i > 0 && (int)blockIdx.x < p.layer[i].first) --i;
-    const StepWeightLayer &l = p.layer[i];
-    const int tiles_k = (l.k + STEP_BN - 1) / STEP_BN;
-    int b = (int)blockIdx.x - l.first;
-    const int slice = b % l.slices;
-    b /= l.slices;
-    const int c0 = (b % tiles_k) * STEP_BN, r0 = (b / tiles_k) * TBM;
-    const int lb = slice * l.rows * l.parts, le = min(p.m, lb + l.rows * l.parts);
+/* Columns of a tile: an accumulator for every eighth slice fits STEP_COLS. */
+__host__ __device__ __forceinline__ int step_width(int count) { return count > 32 ? 32 : 64; }
+
+/* sum_slices adds slices w, w + 8, w + 16, ... of the separate kernel, then
+   those eight sums in order.  Here one CTA takes the slices w, w + 8, ... of
+   a tile, each in an accumulator of its own, and adds them: an eighth of the
+   partial sums to write and read, and the same bits. */
+template <int BN>
+__device__ __forceinline__ void step_weights_tile(uint8_t *tc_smem, const StepWeightLayer &l, int m, int b) {
+    const int tiles_k = (l.k + BN - 1) / BN, slices = min(l.count, 8);
+    const int slice = b % slices;
+    b /= slices;
+    const int c0 = (b % tiles_k) * BN, r0 = (b / tiles_k) * TBM;
+    const int sums = (l.count - slice + 7) / 8, part = l.rows / TBK;
     uint32_t tmem;
-    const bool ok = tc_product<STEP_BN, true, true, STEP_BN * STEP_PARTS>(tc_smem, l.dpre, l.n, l.x, l.k, l.n, l.k, r0,
-                                                                          c0, lb, le, tmem, l.rows / TBK);
+    const bool ok = tc_product<BN, true, true, STEP_COLS>(tc_smem, l.dpre, l.n, l.x, l.k, l.n, l.k, r0, c0,
+                                                          slice * l.rows, m, tmem, sums * part, part, 8 * l.rows);
     const int r = r0 + tc_row();
 #pragma unroll 1
-    for (int j = threadIdx.x >> 7; j < STEP_BN / 16; j += TNT / 128) {
+    for (int j = threadIdx.x >> 7; j < BN / 16; j += TNT / 128) {
         const int c = c0 + j * 16;
         float v[16];
-        tc_row16(tmem, j, le > lb, ok, v);
-        for (int q = 1; lb + q * l.rows < le; ++q) {
+#pragma unroll
+        for (int z = 0; z < 16; ++z) v[z] = 0.0f;
+        for (int q = 0; q < sums; ++q) {
             float u[16];
-            tc_row16(tmem + (uint32_t)(q * STEP_BN), j, true, ok, u);
+            tc_row16(tmem + (uint32_t)(q * BN), j, true, ok, u);
 #pragma unroll
             for (int z = 0; z < 16; ++z) v[z] += u[z];
         }
         if (r >= l.n || c >= l.k) continue;
         tc_store16(l.out + ((size_t)slice * l.n + r) * l.k + c, v);
     }
-    tc_release<STEP_BN * STEP_PARTS>(tmem);
+    tc_release<STEP_COLS>(tmem);
+}
+
+__global__ void __launch_bounds__(TNT) step_weights(const __grid_constant__ StepWeights p) {
+    extern __shared__ __align__(1024) uint8_t tc_smem[];
+    int i = p.layers - 1;
+    while (i > 0 && (int)blockIdx.x < p.layer[i].first) --i;
+    const StepWeightLayer &l = p.layer[i];
+    if (step_width(l.count) == 64) step_weights_tile<64>(tc_smem, l, p.m, (int)blockIdx.x - l.first);
+    else step_weights_tile<32>(tc_smem, l, p.m, (int)blockIdx.x - l.first);
 }
 
 struct StepUpdate {
     AdamwMulti a;                            /* weights and bias of layer i: tensors 2 i, 2 i + 1 */
     const float *dw[STEP_MAX_LAYERS];        /* [slices][n][k] */
-    const float *db[STEP_MAX_LAYERS];        /* [row groups][n] */
+    const float *db[STEP_MAX_LAYERS];        /* [row chunks][n] */
     uint64_t weights;                        /* elements of all weight tensors */
     uint64_t wstart[STEP_MAX_LAYERS + 1];
     int bstart[STEP_MAX_LAYERS + 1];         /* bias columns, in groups of 32 */
     int slices[STEP_MAX_LAYERS];
-    int layers, groups;                      /* row groups of 32 */
+    int layers, chunks;                      /* row chunks of 64 */
     int tie_count, tie_shift;
     const float *loss_part;
     float *loss;
     int m, weight_blocks, bias_blocks;
 };
 
-/* The sum of sum_slices: eight interleaved sums, then those in order. */
+/* The sum of at most eight values in order. */
 __device__ __forceinline__ float sum_eight(const float *p, int count, size_t stride) {
     float s[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) s[q] = 0.0f;
-    for (int z = 0; z < count; z += 8)
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            if (z + q < count) s[q] += p[(size_t)(z + q) * stride];
+    for (int q = 0; q < 8; ++q) s[q] = q < count ? p[(size_t)q * stride] : 0.0f;
     float t = 0.0f;
 #pragma unroll
     for (int q = 0; q < 8; ++q) t += s[q];
@@ -291,7 +310,7 @@ __global__ void __launch_bounds__(256) step_update(const __grid_constant__ StepU
         const int c = (b - p.bstart[k]) * 32 + lane;
         float s = 0.0f;
         if (c < T.cols)
-            for (int z = w; z < p.groups; z += 8) s += p.db[k][(size_t)z * T.cols + c];
+            for (int z = w; z < p.chunks; z += 8) s += p.db[k][(size_t)z * T.cols + c];
         red[w][lane] = s;
         __syncthreads();
         if (w == 0 && c < T.cols) {
@@ -305,9 +324,12 @@ __global__ void __launch_bounds__(256) step_update(const __grid_constant__ StepU
         return;
     }
     /* the loss of each 256 rows from its eight groups' two column halves */
-    const int chunks = (p.m + 255) / 256;
-    for (int i = threadIdx.x; i < chunks; i += 256)
-        p.loss[i] = sum_eight(p.loss_part + 16 * i, 2 * min(8, p.groups - 8 * i), 1);
+    const int groups = (p.m + 31) / 32;
+    for (int i = threadIdx.x; 8 * i < groups; i += 256) {
+        const float *l = p.loss_part + 16 * i;
+        const int n = min(8, groups - 8 * i);
+        p.loss[i] = sum_eight(l, n, 2) + sum_eight(l + 1, n, 2);
+    }
 }
 
 /* Launch behind the previous kernel of the stream, set-up overlapping it. */
@@ -333,22 +355,9 @@ cudaError_t step_launch_tc(void (*kernel)(const P), size_t smem, dim3 grid, cuda
     return e == cudaSuccess ? step_launch(kernel, grid, TNT, smem, st, p) : e;
 }
 
-/* Weight-gradient slices of a layer: the rows per accumulator are those of a
-   slice of mcgb_mlp_linear_bwd_weight, as many to a CTA (STEP_PARTS at most)
-   as leave two CTAs for every SM over the layers' `tiles` tiles. */
-void step_slices(const McgbAdamwTensor &t, int m, int tiles, int &rows, int &parts, int &slices) {
+/* The weight-gradient slices of mcgb_mlp_linear_bwd_weight. */
+void step_slices(const McgbAdamwTensor &t, int m, int &rows, int &count) {
     const int fine = weight_slices(m, t.rows, t.cols, 0);
     rows = ((m + fine - 1) / fine + TBK - 1) / TBK * TBK;
-    const int count = (m + rows - 1) / rows;
-    const int most = 2 * sm_count() / tiles < 1 ? 1 : 2 * sm_count() / tiles;
-    parts = (count + most - 1) / most;
-    parts = parts > STEP_PARTS ? STEP_PARTS : parts;
-    slices = (count + parts - 1) / parts;
-}
-
-int step_tiles(const McgbAdamwTensor *t, int layers) {
-    int tiles = 0;
-    for (int i = 0; i < layers; ++i)
-        tiles += ((t[2 * i].rows + TBM - 1) / TBM) * ((t[2 * i].cols + STEP_BN - 1) / STEP_BN);
-    return tiles;
+    count = (m + rows - 1) / rows;
 }

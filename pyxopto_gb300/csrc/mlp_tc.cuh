@@ -204,21 +204,24 @@ __device__ __forceinline__ void tc_after_previous() {
 }
 
 /* The product of one output tile: rows r0.. of op(A) and c0.. of op(B) over
-   the reduction range [lb, le).  Returns with the accumulator rows 32 (w mod
-   4).. of warp w in those TMEM lanes of `tmem`, and false when a wait ran
-   out.  The reduction starts a new accumulator, BN columns on, every `part`
-   chunks (COLS / BN of them at most). */
+   nch chunks of the reduction range [lb, le), by default all of them.
+   Returns with the accumulator rows 32 (w mod 4).. of warp w in those TMEM
+   lanes of `tmem`, and false when a wait ran out.  Every `part` chunks the
+   range goes on `hop` after the last such start and in a new accumulator, BN
+   columns on (COLS / BN of them at most). */
 template <int BN, bool TA, bool TB, int COLS = BN>
 __device__ __forceinline__ bool tc_product(uint8_t *tc_smem, const bf16 *__restrict__ A, int lda,
                                            const bf16 *__restrict__ B, int ldb, int R, int Cc, int r0, int c0,
-                                           int lb, int le, uint32_t &tmem, int part = 1 << 30) {
+                                           int lb, int le, uint32_t &tmem, int nch = -1, int part = 1 << 30,
+                                           int hop = 0) {
     typedef TcShape<BN> Sh;
     typedef TcStage<TA, TBM> StA;
     typedef TcStage<TB, BN> StB;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(tc_smem);
     const uint32_t bar0 = sbase + Sh::BARS, taddr_slot = sbase + Sh::TADDR;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int nch = le > lb ? (le - lb + TBK - 1) / TBK : 0;
+    if (nch < 0) nch = le > lb ? (le - lb + TBK - 1) / TBK : 0;
+    auto chunk = [&](int i) { return lb + i / part * hop + i % part * TBK; };
 
     if (tid == 0) {
 #pragma unroll
@@ -235,8 +238,8 @@ __device__ __forceinline__ bool tc_product(uint8_t *tc_smem, const bf16 *__restr
     /* the first TC_STAGES chunks go in flight at once */
     for (int i = 0; i < nch && i < TC_STAGES; ++i) {
         const uint32_t st = sbase + i * Sh::STAGE;
-        StA::issue(st, A, lda, R, le, r0, lb + i * TBK);
-        StB::issue(st + TC_A_BYTES, B, ldb, Cc, le, c0, lb + i * TBK);
+        StA::issue(st, A, lda, R, le, r0, chunk(i));
+        StB::issue(st + TC_A_BYTES, B, ldb, Cc, le, c0, chunk(i));
         tc_cp_commit();
     }
     tc_fence_before();
@@ -266,7 +269,7 @@ __device__ __forceinline__ bool tc_product(uint8_t *tc_smem, const bf16 *__restr
             /* refill the stage once its MMAs have read it */
             if (ok) ok = tc_mbar_wait(bar, (uint32_t)(i / TC_STAGES) & 1u, t_end);
             const uint32_t st = sbase + s * Sh::STAGE;
-            const int l0 = lb + (i + TC_STAGES) * TBK;
+            const int l0 = chunk(i + TC_STAGES);
             StA::issue(st, A, lda, R, le, r0, l0);
             StB::issue(st + TC_A_BYTES, B, ldb, Cc, le, c0, l0);
             tc_cp_commit();
