@@ -444,7 +444,9 @@ def surrogate_bench(args):
     seq = BatchedMc.sample_sims(args.seq_profiles + 1, seed=31, packets=(1, 2))
     seq_rate = sequential_plain_mc(seq, 1_000_000)
     value = 65536 / sec
-    launches_per_serve = 4 * ((65536 + sur.mlp.batch - 1) // sur.mlp.batch) + 2
+    # per pass of up to 131072 queries: the input kernel, the layers' GEMMs and
+    # the profile kernel; the judge: batch preparation and batched engine
+    launches_per_serve = (len(sur.mlp.w) + 2) * ((65536 + (1 << 17) - 1) >> 17) + 2
     stat = lambda v: {'median': float(np.median(v)), 'mean': float(np.mean(v)),
                       'p90': float(np.percentile(v, 90))}
     return {'metric': 'profiles/s (surrogate + 1% MC judge, 65536 queries)', 'value': value,
@@ -509,12 +511,13 @@ def mlp_train_bench(args):
     b.record()
     torch.cuda.synchronize()
     ms = a.elapsed_time(b) / (args.steps * inner)
-    # launches per step: the layers' forward GEMMs, the loss gradient, per
-    # layer the activation backward + bias sum and the weight gradient + slice
-    # sum, the input gradients below the top layer, the tied input columns and
-    # one AdamW over every tensor
+    # launches per step: the layers' forward GEMMs (loss and its gradient in
+    # the last), the input gradients below the top layer, the weight gradients
+    # of all layers, and the sums, tied columns and AdamW; with the mma.sync
+    # GEMMs the separate kernels instead
     nl = len(net.w)
-    launches = nl + 1 + 4 * nl + (nl - 1) + (1 if net.split else 0) + 1
+    launches = nl + (nl - 1) + 2 if args.mlp_gemm == 'tcgen05' else \
+        nl + 1 + 4 * nl + (nl - 1) + (1 if net.split else 0) + 1
     flops = 3 * 2 * m * (16 * 256 + 256 * 256 * 2 + 256 * 32)
     return {'metric': 'training profiles/s (MLP 4-256-256-256-30, batch 4096)', 'value': m / (ms / 1e3),
             'unit': 'profiles/s', 'ms_per_step': ms, 'tflops_dense': flops / (ms / 1e3) / 1e12,

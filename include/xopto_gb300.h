@@ -363,14 +363,15 @@ typedef struct McgbRunOptions {
     int32_t track_optical_pathlength;       /* MC_TRACK_OPTICAL_PATHLENGTH     */
     uint32_t block_size;                    /* threads per block (0 = auto);
                                                STATIC scheduling only, the
-                                               DYNAMIC kernels use 128         */
+                                               DYNAMIC kernels choose theirs   */
     uint64_t max_steps_per_packet;          /* 0 = unlimited (2^32 - 1 at most) */
     double deadline_s;                      /* device wall-clock limit, 0=300s */
     int32_t scheduling;                     /* MCGB_SCHED_*                    */
-    uint32_t packets_per_item;              /* DYNAMIC: packets a warp takes
-                                               from the queue at a time, 1-128
-                                               (0 = chosen from the packet
-                                               count and the grid)             */
+    uint32_t packets_per_item;              /* DYNAMIC: most packets a warp
+                                               takes from the queue at a time,
+                                               1-128 (0 = chosen from the packet
+                                               count and the grid); a share of
+                                               what is left near the end       */
     uint64_t seed;                          /* DYNAMIC: stream derivation seed */
     uint64_t packet_offset;                 /* DYNAMIC: index of packet 0      */
 } McgbRunOptions;
@@ -600,7 +601,8 @@ int mcgb_batched_work_size(uint32_t num_sims, uint64_t *bytes);
 
 /* Runs every simulation to completion in one persistent launch (plus a
    small preparation kernel).  Warps take work items of packets_per_item
-   consecutive packets from a device queue and refill idle lanes packet by
+   packets of consecutive queue places (the simulations with the longest-lived
+   packets first, smaller items near the end) from a device queue and refill idle lanes packet by
    packet; packet k of simulation s uses the MWC stream derived from
    (seed, s, k), so the tallies do not depend on the scheduling.
    dev_sims [num_sims]; dev_multipliers [num_multipliers] safe-prime

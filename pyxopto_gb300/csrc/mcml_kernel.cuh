@@ -2,10 +2,12 @@
  * mcml_kernel.cuh - photon-packet transport in a stack of layers
  * (the GB300 counterpart of McKernel, xopto/mcml/kernel/mcml.template.c:346-824).
  *
- * One thread = one random-number stream.  Thread t simulates packets
- * t, t+T, t+2T, ... < N (T = num_streams); when a packet terminates the thread
- * launches its next packet inside the same loop iteration, so a warp keeps
- * all lanes busy until the lanes run out of packets.
+ * Static kernels: one thread = one random-number stream.  Thread t simulates
+ * packets t, t+T, t+2T, ... < N (T = num_streams); when a packet terminates
+ * the thread launches its next packet inside the same loop iteration.
+ * Dynamic kernels: one packet = one stream.  Warps take packet numbers from a
+ * queue for their idle lanes every 16 steps, and pass on their last packets
+ * once it is empty (work_share.cuh).
  *
  * The layer table is rebuilt in shared memory as 16-byte records read with
  * vector loads (divergent per-lane layer indices hit distinct shared-memory
