@@ -57,12 +57,12 @@ L2_FLUSH_BYTES = 256 << 20
 # fraction of issue slots in use (smsp__issue_active), the resource that
 # bounds this kernel.
 PROFILED_TRAFFIC = {
-    ('c2_skin_gk_fluence', 'fast', 'dynamic'): (7.74e6, 'profiles/mcml_dynamic_kernel_c2_skin_gk_fluence.md'),
-    ('c3_vox_skin_vessel', 'fast', 'dynamic'): (1.80e10, 'profiles/mcvox_dynamic_kernel_c3_skin_vessel_200cubed.md'),
+    ('c2_skin_gk_fluence', 'fast', 'dynamic'): (7.76e6, 'profiles/mcml_dynamic_kernel_c2_skin_gk_fluence.md'),
+    ('c3_vox_skin_vessel', 'fast', 'dynamic'): (1.81e10, 'profiles/mcvox_dynamic_kernel_c3_skin_vessel_200cubed.md'),
 }
 PROFILED_ISSUE_ACTIVE = {
-    ('c2_skin_gk_fluence', 'fast', 'dynamic'): (0.875, 'profiles/mcml_dynamic_kernel_c2_skin_gk_fluence.md'),
-    ('c3_vox_skin_vessel', 'fast', 'dynamic'): (0.867, 'profiles/mcvox_dynamic_kernel_c3_skin_vessel_200cubed.md'),
+    ('c2_skin_gk_fluence', 'fast', 'dynamic'): (0.882, 'profiles/mcml_dynamic_kernel_c2_skin_gk_fluence.md'),
+    ('c3_vox_skin_vessel', 'fast', 'dynamic'): (0.870, 'profiles/mcvox_dynamic_kernel_c3_skin_vessel_200cubed.md'),
 }
 # L2 atomic-unit use of the transport kernel's 64-bit tally atomics, from a
 # medium-case ncu capture (one kernel, one launch, 2e7 packets): the share of
@@ -71,12 +71,12 @@ PROFILED_ISSUE_ACTIVE = {
 # per interaction step (lts__t_requests_op_red), and the L2 throughput.
 PROFILED_L2_ATOMICS = {
     ('c2_skin_gk_fluence', 'fast', 'dynamic'): (
-        {'atomic_unit_active_pct': 14.66, 'red_requests_per_packet': 436.6,
-         'red_requests_per_ref_step': 0.484, 'lts_throughput_pct': 21.98},
+        {'atomic_unit_active_pct': 17.64, 'red_requests_per_packet': 433.8,
+         'red_requests_per_ref_step': 0.480, 'lts_throughput_pct': 26.45},
         'profiles/mcml_dynamic_kernel_c2_skin_gk_fluence.md'),
     ('c3_vox_skin_vessel', 'fast', 'dynamic'): (
-        {'atomic_unit_active_pct': 12.22, 'red_requests_per_packet': 300.1,
-         'red_requests_per_ref_step': 0.370, 'lts_throughput_pct': 24.04},
+        {'atomic_unit_active_pct': 12.58, 'red_requests_per_packet': 297.6,
+         'red_requests_per_ref_step': 0.367, 'lts_throughput_pct': 24.34},
         'profiles/mcvox_dynamic_kernel_c3_skin_vessel_200cubed.md'),
 }
 # DRAM traffic of the voxel fluence (same capture): dram__bytes_read +
@@ -84,7 +84,7 @@ PROFILED_L2_ATOMICS = {
 # fluence tally's atomics; the tally itself is read once).
 PROFILED_HBM = {
     ('c3_vox_skin_vessel', 'fast', 'dynamic'): (
-        {'gbs': 41.7, 'bytes_per_packet': 180.2},
+        {'gbs': 43.1, 'bytes_per_packet': 180.6},
         'profiles/mcvox_dynamic_kernel_c3_skin_vessel_200cubed.md'),
 }
 HBM_FALLBACK_GBS = 6800.0
