@@ -907,7 +907,9 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
             bool done;
             if (DEFER) {
                 done = mcml_step_weight<PF, FLU, XTRA, true>(c, b, x, s, rng, fcache);
-                done = mcml_step_end<XTRA, XTRA || !SIMPLE>(c, b, x, s, status, done);
+                /* a held step ends with its hit: before it the packet has not
+                   moved, and its launch point may lie beyond rmax */
+                if (s.pend < 0.0f) done = mcml_step_end<XTRA, XTRA || !SIMPLE>(c, b, x, s, status, done);
             } else {
                 done = mcml_step<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status);
             }
