@@ -722,8 +722,9 @@ int mcgb_mlp_adamw_multi(const McgbAdamwTensor *tensors, int count, float lr, fl
    their grad arrays receive the gradients.  h[i] and pre[i] receive layer
    i's output and pre-activation, dpre[i] the gradient of the latter; loss
    [ceil(m / 256)] the loss of every 256 rows.  x [m, cols of layer 0] bf16
-   and target [m, 32] are 16-byte aligned, scratch holds
-   mcgb_mlp_train_scratch(tensors, layers, m) floats.  tcgen05 path only. */
+   and target [m, 32] are 16-byte aligned, scratch holds scratch_size floats,
+   at least mcgb_mlp_train_scratch(tensors, layers, m); the answer for a
+   batch also serves every smaller m.  tcgen05 path only. */
 typedef struct McgbMlpStep {
     const McgbAdamwTensor *tensors;                 /* host array, 2 * layers */
     const uint16_t *x;
@@ -738,6 +739,7 @@ typedef struct McgbMlpStep {
     int32_t layers, m, nv, mode;
     int32_t tie_count, tie_shift, step, reserved;
     float scale, lr, beta1, beta2, eps, reserved2;
+    uint64_t scratch_size;                          /* floats of scratch      */
 } McgbMlpStep;
 
 int mcgb_mlp_train_step(const McgbMlpStep *step, void *stream);

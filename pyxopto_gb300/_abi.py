@@ -168,7 +168,8 @@ class McgbMlpStep(C.Structure):
                 ('dpre', C.c_void_p * (ADAMW_MAX_TENSORS // 2)),
                 ('layers', i32), ('m', i32), ('nv', i32), ('mode', i32),
                 ('tie_count', i32), ('tie_shift', i32), ('step', i32), ('reserved', i32),
-                ('scale', f32), ('lr', f32), ('beta1', f32), ('beta2', f32), ('eps', f32), ('reserved2', f32)]
+                ('scale', f32), ('lr', f32), ('beta1', f32), ('beta2', f32), ('eps', f32), ('reserved2', f32),
+                ('scratch_size', u64)]
 
 
 class McgbMlpPredict(C.Structure):

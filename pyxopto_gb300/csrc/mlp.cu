@@ -624,15 +624,16 @@ int mcgb_mlp_predict(const McgbMlpPredict *p, void *stream) {
     return check_launch("mlp profiles");
 }
 
+/* Counts weight_slices, which only grows with m, and not the step's slices:
+   those round their rows up to 64 and so can be fewer for a larger m. */
 uint64_t mcgb_mlp_train_scratch(const McgbAdamwTensor *tensors, int layers, int m) {
     if (!tensors || layers < 1 || layers > STEP_MAX_LAYERS || m <= 0) return 0;
     const uint64_t groups = (uint64_t)(m + 31) / 32, chunks = (uint64_t)(m + 63) / 64;
     uint64_t n = (2 * groups + 3) / 4 * 4;
     for (int i = 0; i < layers; ++i) {
-        int rows, count;
-        step_slices(tensors[2 * i], m, rows, count);
-        n += (uint64_t)(count < 8 ? count : 8) * tensors[2 * i].rows * tensors[2 * i].cols +
-             chunks * (uint64_t)tensors[2 * i].rows;
+        const McgbAdamwTensor &t = tensors[2 * i];
+        const int most = weight_slices(m, t.rows, t.cols, 0);
+        n += (uint64_t)(most < 8 ? most : 8) * t.rows * t.cols + chunks * (uint64_t)t.rows;
     }
     return n;
 }
@@ -661,6 +662,10 @@ int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
     const uintptr_t all = (uintptr_t)s->x | (uintptr_t)s->x_copy | (uintptr_t)s->target |
                           (uintptr_t)s->scratch;
     if (all & 15u) return fail(MCGB_E_INVALID, "train_step operands must be 16-byte aligned");
+    const uint64_t need = mcgb_mlp_train_scratch(t, L, m);
+    if (s->scratch_size < need)
+        return fail(MCGB_E_SIZE, "train_step scratch of %llu floats, %llu needed for %d rows",
+                    (unsigned long long)s->scratch_size, (unsigned long long)need, m);
 
     cudaStream_t st = (cudaStream_t)stream;
     int rows[STEP_MAX_LAYERS], count[STEP_MAX_LAYERS], slices[STEP_MAX_LAYERS];

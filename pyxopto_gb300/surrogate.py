@@ -243,6 +243,7 @@ class Mlp:
             nscr = int(self.lib.mcgb_mlp_train_scratch(s.tensors, nl, self.batch))
             self._step_scratch = self.torch.empty((max(nscr, 1),), dtype=self.torch.float32, device='cuda')
             s.scratch, s.loss = self._step_scratch.data_ptr(), self.loss_part.data_ptr()
+            s.scratch_size = self._step_scratch.numel()
             for i in range(nl):
                 s.h[i], s.pre[i], s.dpre[i] = (v.data_ptr() for v in (self.h[i + 1], self.pre[i], self.dpre[i]))
             s.layers = nl
