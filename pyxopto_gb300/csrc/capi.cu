@@ -240,7 +240,7 @@ int make_shape(int medium, int math, uint32_t block_size, uint32_t num_streams, 
     if (s->block > 256 || (s->block % 32) != 0)
         return fail(MCGB_E_INVALID, "block size %u must be a multiple of 32 and <= 256", s->block);
     s->grid = (num_streams + s->block - 1) / s->block;
-    s->lut_in_smem = (b->fp_lut && b->fp_lut_size > 0 && b->fp_lut_size <= 24576) ? 1 : 0;
+    s->lut_in_smem = (b->fp_lut && b->fp_lut_size > 0 && b->fp_lut_size <= MCGB_SMEM_TABLE_FLOATS) ? 1 : 0;
     s->dyn_smem = s->lut_in_smem ? (size_t)b->fp_lut_size * sizeof(float) : 0;
     double d = deadline_s > 0.0 ? deadline_s : 300.0;
     s->deadline_ns = (uint64_t)(d * 1e9);

@@ -6,6 +6,9 @@
 #include <cuda_runtime.h>
 #include "../../include/xopto_gb300.h"
 
+/* Longest float table that the kernels stage in shared memory (96 KB). */
+#define MCGB_SMEM_TABLE_FLOATS 24576u
+
 struct LaunchShape {
     unsigned grid;
     unsigned block;

@@ -120,9 +120,13 @@ cudaError_t MCGB_LAUNCH(const MCGB_CFG &cfg, const McgbBuffers &buf, cudaStream_
     const void *k = select(sched, cfg.pf_kind, cfg.opt.method, cfg.fluence.kind != MCGB_FLUENCE_NONE,
                            xtra, simple_source(cfg.source.kind) && !rmax);
     if (!k) return cudaErrorInvalidValue;
-    if (shape.dyn_smem > 48 * 1024) {
+    /* The 48 KB that need no opt-in cover the kernel's own tables (7.5 KB
+       layered, 19 KB voxelized, dynamic) and the table passed here together.
+       The opt-in is for the largest table, so that runs of other tables in
+       other threads may set it at the same time. */
+    if (shape.dyn_smem > 0) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)shape.dyn_smem);
+                                             (int)(MCGB_SMEM_TABLE_FLOATS * sizeof(float)));
         if (e != cudaSuccess) return e;
     }
     unsigned grid = shape.grid, block = shape.block;
