@@ -382,15 +382,18 @@ class Surrogate:
     def predict(self, mua, musr, g, n):
         """Reflectance profiles [M, bins] for the given optical properties.
         The inputs and the exponential are computed on the device in double
-        precision."""
+        precision; networks of more than eight layers go layer by layer,
+        with both on the host."""
         import torch
         m = len(np.asarray(mua))
+        nb, net = self.raxis.n, self.mlp
+        if m == 0 or nb > OUT_PAD:
+            raise ValueError('predict needs at least one query and at most {} bins'.format(OUT_PAD))
+        if len(net.w) > _abi.ADAMW_MAX_TENSORS // 2:
+            return self._predict_layers(features(mua, musr, g, n))
         q = np.empty((4, m))
         for i, c in enumerate((mua, musr, g, n)):
             q[i] = c
-        nb, net = self.raxis.n, self.mlp
-        if m == 0 or nb > OUT_PAD or not 1 <= len(net.w) <= _abi.ADAMW_MAX_TENSORS // 2:
-            raise ValueError('predict needs at least one query and at most {} bins'.format(OUT_PAD))
         p = _abi.McgbMlpPredict()
         nl = p.layers = len(net.w)
         for i in range(nl):
@@ -414,6 +417,20 @@ class Surrogate:
             p.queries, p.m, p.profiles = part.data_ptr(), part.shape[1], out[s:].data_ptr()
             _lib.check(net.lib.mcgb_mlp_predict(C.byref(p), net._stream()))
         return out.cpu().numpy()
+
+    def _predict_layers(self, x):
+        """predict() of a network of any number of layers."""
+        m = len(x)
+        mp = (m + 7) // 8 * 8
+        xp = np.zeros((mp, IN_PAD), np.float32)
+        xp[:m] = x
+        xd = split_bf16(xp)
+        out = []
+        for s in range(0, mp, self.mlp.batch):
+            z = self.mlp.forward(xd[s:s + self.mlp.batch], store=False)
+            out.append(z[:, :self.raxis.n].cpu().numpy().astype(np.float64))
+        z = np.concatenate(out)[:m]
+        return np.exp(self.mu[None, :] + self.scale * z)
 
     # ------------------------------------------------------ weights
     def save(self, path):
