@@ -389,7 +389,7 @@ class Surrogate:
         nb, net = self.raxis.n, self.mlp
         if m == 0 or nb > OUT_PAD:
             raise ValueError('predict needs at least one query and at most {} bins'.format(OUT_PAD))
-        if len(net.w) > _abi.ADAMW_MAX_TENSORS // 2:
+        if len(net.w) > _abi.ADAMW_MAX_TENSORS // 2 or np.shape(self.mu) != (nb,) or np.ndim(self.scale):
             return self._predict_layers(features(mua, musr, g, n))
         q = np.empty((4, m))
         for i, c in enumerate((mua, musr, g, n)):
@@ -419,7 +419,7 @@ class Surrogate:
         return out.cpu().numpy()
 
     def _predict_layers(self, x):
-        """predict() of a network of any number of layers."""
+        """predict() for any network and normalisation that broadcasts."""
         m = len(x)
         mp = (m + 7) // 8 * 8
         xp = np.zeros((mp, IN_PAD), np.float32)

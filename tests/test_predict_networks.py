@@ -1,4 +1,5 @@
-"""Surrogate.predict of networks that the one-call path does not take."""
+"""Surrogate.predict of networks and normalisations that the one-call path
+does not take."""
 import numpy as np
 import pytest
 
@@ -38,3 +39,20 @@ def test_deep_networks(cuda, lib, hidden, m):
     x[:m] = features(*q)
     z = net.forward(split_bf16(x))[:m, :30].cpu().numpy().astype(np.float64)
     assert np.max(np.abs(got / np.exp(sur.mu + sur.scale * z) - 1.0)) < 1e-3
+
+
+@pytest.mark.gpu
+def test_normalisation_of_another_length_is_refused(cuda, lib):
+    sur = _surrogate((4, 64, 30))
+    sur.mu = sur.mu[:20]
+    with pytest.raises(ValueError):
+        sur.predict(*_queries(9))
+
+
+@pytest.mark.gpu
+def test_normalisation_per_bin(cuda, lib):
+    sur = _surrogate((4, 64, 30))
+    q = _queries(9)
+    one = sur.predict(*q)
+    sur.scale = np.full(30, sur.scale)
+    assert np.max(np.abs(sur.predict(*q) / one - 1.0)) < 1e-3
