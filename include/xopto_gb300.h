@@ -752,7 +752,8 @@ uint64_t mcgb_mlp_train_scratch(const McgbAdamwTensor *tensors, int layers, int 
    by their logarithm.  Device pointers but for the struct itself; x [rows,
    16], h[0] and h[1] [rows, widest hidden layer or 32] and z [rows, 32] are
    scratch for rows = m rounded up to a multiple of 8.  widths[0] = 16,
-   widths[layers] = 32. */
+   widths[layers] = 32.  At most 65535 * 128 queries (65535 * 64 with the
+   mma.sync GEMMs) in one call, as in a training step. */
 typedef struct McgbMlpPredict {
     const uint16_t *w[MCGB_ADAMW_MAX_TENSORS / 2];
     const float *b[MCGB_ADAMW_MAX_TENSORS / 2];

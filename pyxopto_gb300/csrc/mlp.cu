@@ -403,6 +403,12 @@ int sm_count() {
     return n;
 }
 
+/* Rows that one launch reaches: a row of tiles per grid.y step. */
+int rows_fit(int m) {
+    const int most = 65535 * (g_gemm_path == 0 ? TBM : BM);
+    return m <= most ? MCGB_OK : fail(MCGB_E_SIZE, "%d rows, at most %d in one call", m, most);
+}
+
 /* Reduction slices of the weight gradient for a GEMM path: enough that the
    grid of output tiles times slices covers every SM twice, each slice at
    least one k-step of rows, at most 64 slices. */
@@ -593,9 +599,11 @@ int mcgb_mlp_adamw_multi(const McgbAdamwTensor *tensors, int count, float lr, fl
 }
 
 int mcgb_mlp_predict(const McgbMlpPredict *p, void *stream) {
-    if (!p || p->layers < 1 || p->layers > MCGB_ADAMW_MAX_TENSORS / 2 || p->m < 1 || p->m > (1 << 24) ||
+    if (!p || p->layers < 1 || p->layers > MCGB_ADAMW_MAX_TENSORS / 2 || p->m < 1 ||
         p->bins < 1 || p->bins > 32 || !p->queries || !p->mu || !p->x || !p->h[0] || !p->h[1] || !p->z || !p->profiles)
         return fail(MCGB_E_INVALID, "bad predict arguments");
+    const int fit = rows_fit(p->m);
+    if (fit) return fit;
     const int L = p->layers, m = p->m, rows = (m + 7) / 8 * 8;
     if (p->widths[0] != 16 || p->widths[L] != 32)
         return fail(MCGB_E_UNSUPPORTED, "predict takes 16 input and 32 output columns");
@@ -645,6 +653,8 @@ int mcgb_mlp_train_step(const McgbMlpStep *s, void *stream) {
     const int L = s->layers, m = s->m;
     const McgbAdamwTensor *t = s->tensors;
     if (g_gemm_path != 0) return fail(MCGB_E_UNSUPPORTED, "train_step runs on the tcgen05 GEMM path only");
+    const int fit = rows_fit(m);
+    if (fit) return fit;
     for (int i = 0; i < L; ++i) {
         const McgbAdamwTensor &w = t[2 * i], &b = t[2 * i + 1];
         int r = shape_ok(m, w.rows, w.cols);
