@@ -735,10 +735,20 @@ mcvox_transport_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuff
 }
 
 /* Threads per block of the dynamic kernel: the warps that merge their last
-   packets.  The plain Line and GaussianBeam kernels take 64 registers by
-   themselves; with a minimum of four blocks they lost 4 % on the skin and
-   vessel grid, with a minimum of one (76 registers) 30 %. */
+   packets.  The plain Line and GaussianBeam kernels mostly take 64 registers
+   by themselves (32 warps an SM); with a minimum of four blocks they lost 4 %
+   on the skin and vessel grid, with a minimum of one (76 registers) 30 %.
+   The others take 57 to 80 (24 to 32 warps), but the EXACT kernels with a
+   fluence grid, the optional features and every source 104 to 107: 16 warps.
+   A minimum of three blocks brings those to 80 at most: fluence rate of the
+   vessel grid from a UniformBeam, 1e6 packets with rmax 10.1 -> 9.1 ms, 5e5
+   without 9.96 -> 9.6 ms.  The other variants lose by it or are as they were
+   (1e6 packets of a UniformBeam, FAST 5.8 -> 6.1 ms, EXACT 11.3 -> 11.6). */
 #define MV_BLOCK 256
+template <bool FLU, bool XTRA, bool SIMPLE>
+constexpr int mv_min_blocks() {
+    return !MCGB_FAST_MATH && FLU && XTRA && !SIMPLE ? 3 : 0;   /* 0 = none */
+}
 
 /* Everything of a packet that moves between warps (work_share.cuh). */
 template <bool XTRA, class IO>
@@ -757,7 +767,7 @@ typedef WsExchange<23, MV_BLOCK / 32, 2, 2> MvExchange;
 
 /* DYNAMIC scheduling (per-packet streams, warp refill). */
 template <int PF, int METHOD, bool FLU, bool XTRA, bool SIMPLE>
-__global__ void __launch_bounds__(MV_BLOCK)
+__global__ void __launch_bounds__(MV_BLOCK, mv_min_blocks<FLU, XTRA, SIMPLE>())
 mcvox_dynamic_kernel(const __grid_constant__ McgbMcvoxConfig c, const McgbBuffers b,
                      uint64_t deadline_ns, int lut_in_smem, uint32_t packets_per_item) {
     __shared__ MvSmem sm;
