@@ -367,11 +367,12 @@ typedef struct McgbRunOptions {
     uint64_t max_steps_per_packet;          /* 0 = unlimited (2^32 - 1 at most) */
     double deadline_s;                      /* device wall-clock limit, 0=300s */
     int32_t scheduling;                     /* MCGB_SCHED_*                    */
-    uint32_t packets_per_item;              /* DYNAMIC: most packets a warp
-                                               takes from the queue at a time,
-                                               1-128 (0 = chosen from the packet
-                                               count and the grid); a share of
-                                               what is left near the end       */
+    uint32_t packets_per_item;              /* DYNAMIC: packets a warp takes
+                                               from the queue at a time, 1-128,
+                                               as many at every visit; 0 = up
+                                               to 128, by the packets left and
+                                               the grid, down to the idle lanes
+                                               near the end                    */
     uint64_t seed;                          /* DYNAMIC: stream derivation seed */
     uint64_t packet_offset;                 /* DYNAMIC: index of packet 0      */
 } McgbRunOptions;

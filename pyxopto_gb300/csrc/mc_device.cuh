@@ -349,7 +349,8 @@ MCGB_DEV float pf_sample(const float4 &pf0, const float4 &pf1, const float *lut,
         float e = pf0.z * em_log_normal(base);
         float tmp = pf1.y - em_exp_mid(e);
         float cos_theta = em_quot(tmp, pf1.z, em_recip(pf1.z));
-        /* tmp is 0 or at least 2^-24 of its larger term, below 2^117 */
+        /* |e| <= 40 keeps exp(e) below 2^58, and with it the numerator tmp
+           in em_quot's range: it is 0 or at least 2^-24 of its larger term */
         if (__float_as_uint(base) - 0x00800000u < 0x7f000000u && fabsf(e) <= 40.0f && pf0.y != 0.0f &&
             fabsf(pf1.z) >= EM_LO) {
             rng = next;
