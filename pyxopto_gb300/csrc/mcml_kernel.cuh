@@ -592,11 +592,16 @@ static __device__ __forceinline__ bool mcml_interact(const McgbMcmlConfig &c, Ml
    About one step in a hundred hits a boundary, so little is computed in
    vain, and a warp pays for it anyway while one of its lanes scatters.  FAST
    math: 1e7 packets of the skin stack 53.7 -> 49.1 ms, 1e6 of the slab
-   1.90 -> 1.70 ms. */
-template <int PF, bool FLU, bool XTRA, bool DEFER = false>
+   1.90 -> 1.70 ms.
+   With DEFER a step that reaches a boundary is held (s.pend) and the others
+   are ended here: a held step must not be, since the packet has not moved
+   and its launch point may lie beyond rmax.  On its way out of the function
+   a held step skips the test for nothing; testing s.pend after the call cost
+   the fibre 2 %. */
+template <int PF, bool FLU, bool XTRA, bool DEFER, bool RMAX>
 static __device__ __forceinline__ bool mcml_step_weight(const McgbMcmlConfig &c, const McgbBuffers &b,
                                                         const MlCtx &x, MlPacket &s, Rng &rng,
-                                                        FluenceCache &fcache) {
+                                                        FluenceCache &fcache, uint32_t &status) {
     const MlLayer &cl = x.L[s.layer];
     const float4 g0 = cl.g0;   /* top, bottom, step factor, mua_inv_mut */
     ++s.steps;
@@ -622,7 +627,8 @@ static __device__ __forceinline__ bool mcml_step_weight(const McgbMcmlConfig &c,
     s.pos.y = s.pos.y + s.dir.y * step;
     s.pos.z = s.pos.z + s.dir.z * step;
     if (XTRA && x.track_opl) s.opl += cl.g1.x * step;
-    return mcml_interact<FLU, XTRA>(c, s, rng, srng, sdir, g0.w, cl.g1.y, fcache);
+    bool done = mcml_interact<FLU, XTRA>(c, s, rng, srng, sdir, g0.w, cl.g1.y, fcache);
+    return DEFER ? mcml_step_end<XTRA, RMAX>(c, b, x, s, status, done) : done;
 }
 
 /* The rest of a step whose path (s.pend) reaches a boundary.  Kept apart, so
@@ -658,7 +664,7 @@ static __device__ __forceinline__ bool mcml_step(const McgbMcmlConfig &c, const 
                                                  const MlCtx &x, MlPacket &s, Rng &rng,
                                                  FluenceCache &fcache, uint32_t &status) {
     if (METHOD == MCGB_METHOD_ALBEDO_WEIGHT) {
-        bool done = mcml_step_weight<PF, FLU, XTRA>(c, b, x, s, rng, fcache);
+        bool done = mcml_step_weight<PF, FLU, XTRA, false, RMAX>(c, b, x, s, rng, fcache, status);
         return mcml_step_end<XTRA, RMAX>(c, b, x, s, status, done);
     }
     const MlLayer *L = x.L;
@@ -906,10 +912,7 @@ mcml_dynamic_kernel(const __grid_constant__ McgbMcmlConfig c, const McgbBuffers 
             if (!active || (DEFER && s.pend >= 0.0f)) continue;
             bool done;
             if (DEFER) {
-                done = mcml_step_weight<PF, FLU, XTRA, true>(c, b, x, s, rng, fcache);
-                /* a held step ends with its hit: before it the packet has not
-                   moved, and its launch point may lie beyond rmax */
-                if (s.pend < 0.0f) done = mcml_step_end<XTRA, XTRA || !SIMPLE>(c, b, x, s, status, done);
+                done = mcml_step_weight<PF, FLU, XTRA, true, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status);
             } else {
                 done = mcml_step<PF, METHOD, FLU, XTRA, XTRA || !SIMPLE>(c, b, x, s, rng, fcache, status);
             }
